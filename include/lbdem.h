@@ -413,6 +413,19 @@ int lbdem_dem_launches_last(void);
  *            blocks, which also share the GPU with a step on another stream. */
 int lbdem_dem_substeps(lbdem_dem *D, int32_t nsub, void *stream);
 
+/* The same sub-steps with a workspace: one launch in which a particle waits
+ * for the particles it can touch instead of for the whole grid after every
+ * phase (contact forces on both partners are evaluated by both, without
+ * atomics; same contact sets and states, the contact slots' order may differ).
+ * work: LBDEM_DEM_FLOW_BYTES(n) of 256-byte aligned device memory, zeroed once
+ * by the caller and kept by it between calls, for one solver; D->sync must be
+ * zeroed once too.  Where the form does not apply (a short periodic axis, more
+ * particles than one resident wave holds, a single sub-step of many particles,
+ * no workspace, LBDEM_DEM_KERNELS set in the environment) this is
+ * lbdem_dem_substeps. */
+#define LBDEM_DEM_FLOW_BYTES(n) (256 + 512 * (size_t)(n))
+int lbdem_dem_substeps_flow(lbdem_dem *D, int32_t nsub, void *work, void *stream);
+
 /* FP64 totals over the updated (non-skipped) cells of population buffer
  * f[buf]: out[0] = sum of rho, out[1..3] = sum of momentum.  Valid in either
  * state of the buffer (post-stream or post-collision: streaming conserves

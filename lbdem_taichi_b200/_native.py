@@ -21,6 +21,7 @@ ABI_VERSION = 4        # LBDEM_ABI_VERSION of include/lbdem.h
 F32, F16, BF16 = 0, 1, 2
 LINK_FLUID = 1 << 20   # LBDEM_LINK_FLUID: the link mask of every cell of an all-FLUID lattice
 SMAG_OFF, SMAG_REFERENCE, SMAG_LOCAL = 0, 1, 2
+DEM_FLOW_BYTES = (256, 512)   # LBDEM_DEM_FLOW_BYTES: fixed part, per particle
 SUM_BLOCKS = 1184
 SUM_PARTIALS = 4 * SUM_BLOCKS
 
@@ -95,6 +96,7 @@ EXPORTS = {
     "lbdem_psc_decode": ([vp, vp, vp, vp, vp, vp, vp], C.c_int),
     "lbdem_dem_bin": ([vp, vp], C.c_int),
     "lbdem_dem_substeps": ([vp, C.c_int32, vp], C.c_int),
+    "lbdem_dem_substeps_flow": ([vp, C.c_int32, vp, vp], C.c_int),
     "lbdem_global_sums_f64": ([vp, C.c_int32, vp, vp, vp], C.c_int),
     "lbdem_global_sums_f64_noalloc": ([vp, C.c_int32, vp, vp], C.c_int),
     "lbdem_psc_map_smooth": ([vp, vp, vp, vp, vp], C.c_int),
@@ -172,7 +174,7 @@ def call(name: str, *args):
     if pre is not None:
         _launches[0] += pre
     else:
-        _launches[0] += (load().lbdem_dem_launches_last() if name == "lbdem_dem_substeps"
+        _launches[0] += (load().lbdem_dem_launches_last() if name.startswith("lbdem_dem_substeps")
                          else KERNELS_PER_CALL.get(name, 0))
     if name == "lbdem_psc_step_phase" and args[8]:
         _launches[0] += 1     # a launch sized from an estimate is followed by the one that takes the rest

@@ -32,6 +32,33 @@ struct M3 {
     double m[3][3];
 };
 
+// Reciprocal and square roots without branches: the hardware's approximation
+// (PTX rcp.approx / rsqrt.approx.ftz.f64, about 22 bits) and two Newton-Raphson
+// steps.  A contact has half a dozen of them, one after another in a chain that
+// nothing hides, and the library forms branch for special values, so that not
+// even independent ones overlap.  Arguments here are squared lengths, radii,
+// masses and stiffnesses: positive and far from the ends of the range; a root
+// of less than 1e-290 is 0.  Against the library's results over 1e-30 .. 1e30:
+// at most 1 ulp (rcp64) and 1 ulp (sqrt64) apart.
+__device__ __forceinline__ double rcp64(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    r = fma(r, fma(-x, r, 1.0), r);
+    return fma(r, fma(-x, r, 1.0), r);
+}
+__device__ __forceinline__ double rsqrt64(double x) {
+    double r;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    r = fma(0.5 * r, fma(-x * r, r, 1.0), r);
+    return fma(0.5 * r, fma(-x * r, r, 1.0), r);
+}
+// root of x given r = rsqrt64(x)
+__device__ __forceinline__ double sqrt64(double x, double r) {
+    const double s = x * r;
+    return x > 1e-290 ? fma(0.5 * r, fma(-s, s, x), s) : (x == x ? 0.0 : x);
+}
+__device__ __forceinline__ double sqrt64(double x) { return sqrt64(x, rsqrt64(x)); }
+
 __device__ __forceinline__ void cross3(const double *a, const double *b, double *o) {
     const double t0 = a[1] * b[2] - a[2] * b[1], t1 = a[2] * b[0] - a[0] * b[2], t2 = a[0] * b[1] - a[1] * b[0];
     o[0] = t0; o[1] = t1; o[2] = t2;
@@ -41,6 +68,10 @@ __device__ __forceinline__ void mv(const M3 &M, const double *v, double *o) {
     double t[3];
     for (int r = 0; r < 3; ++r) t[r] = M.m[r][0] * v[0] + M.m[r][1] * v[1] + M.m[r][2] * v[2];
     o[0] = t[0]; o[1] = t[1]; o[2] = t[2];
+}
+// R^T v: the inverse of a rotation (the reference inverts the matrix)
+__device__ __forceinline__ void mtv(const M3 &M, const double *v, double *o) {
+    for (int r = 0; r < 3; ++r) o[r] = M.m[0][r] * v[0] + M.m[1][r] * v[1] + M.m[2][r] * v[2];
 }
 __device__ M3 inv3(const M3 &A) {
     const double(*a)[3] = A.m;
@@ -61,12 +92,12 @@ __device__ M3 rot_to_x(const double *a) {
     const double b[3] = {1.0, 0.0, 0.0};
     double v[3];
     cross3(a, b, v);
-    const double s = sqrt(dot3(v, v));
+    const double s2 = dot3(v, v);
     const double c = dot3(a, b);
     M3 R;
     for (int i = 0; i < 3; ++i)
         for (int j = 0; j < 3; ++j) R.m[i][j] = 0.0;
-    if (s < 1e-12) {
+    if (s2 < 1e-24) {
         if (c > 0.0) {
             R.m[0][0] = R.m[1][1] = R.m[2][2] = 1.0;
         } else {
@@ -74,7 +105,7 @@ __device__ M3 rot_to_x(const double *a) {
         }
     } else {
         const double vx[3][3] = {{0.0, -v[2], v[1]}, {v[2], 0.0, -v[0]}, {-v[1], v[0], 0.0}};
-        const double coef = (1.0 - c) / (s * s);
+        const double coef = (1.0 - c) * rcp64(s2);
         for (int r = 0; r < 3; ++r)
             for (int q = 0; q < 3; ++q) {
                 double acc = 0.0;
@@ -92,10 +123,10 @@ struct DemArgs {
     int ncell;
     int parity;
     // Hertz constants of a contact, [0] particle-particle, [1] particle-wall
-    // (hertz.py:45-97, 99-153: effective Young's and shear moduli, damping
-    // ratio from the restitution), computed once per launch on the host in the
-    // reference's operation order instead of once per contact
-    double hz_ys[2], hz_gs[2], hz_beta[2];
+    // (hertz.py:45-97, 99-153), computed once per launch on the host: with
+    // x = sqrt(Rs delta) and y = sqrt(x ms), stiffnesses kn x and kt x,
+    // dampings gn y and gt y
+    double hz_kn[2], hz_kt[2], hz_gn[2], hz_gt[2];
 };
 
 __device__ __forceinline__ int cell_index(const lbdem_dem &d, int cx_, int cy_, int cz_) {
@@ -133,9 +164,16 @@ __global__ void k_bin(const __grid_constant__ DemArgs A) {
 
 // ------------------------------- contact laws ------------------------------
 // hertz.py:45-97 / linear.py:43-101 (particle-particle), hertz.py:99-153 /
-// linear.py:103-152 (particle-wall).  `wall` selects the wall variant.
-__device__ void contact_force(const DemArgs &A, double rad_i, double mass_i, double rad_j, double mass_j, bool wall,
-                              double *shear, double delta_n, const double *vc, double *F) {
+// linear.py:103-152 (particle-wall).  `wall` selects the wall variant; Rs and
+// ms are the effective radius and mass (pair_effective).  The damping factors
+// of both directions share one root (DemArgs).
+__device__ __forceinline__ void pair_effective(double rad_i, double rad_j, double mass_i, double mass_j, double &Rs,
+                                               double &ms) {
+    Rs = rad_i * rad_j * rcp64(rad_i + rad_j);
+    ms = mass_i * mass_j * rcp64(mass_i + mass_j);
+}
+__device__ __forceinline__ void contact_force(const DemArgs &A, double Rs, double ms, bool wall, double *shear,
+                                              double delta_n, const double *vc, double *F) {
     const lbdem_dem &d = A.d;
     const double gap = -1 * delta_n;
     const double dt = d.dt;
@@ -143,55 +181,40 @@ __device__ void contact_force(const DemArgs &A, double rad_i, double mass_i, dou
     inc[0] = 0.0;
     double kt, gt, F0, mu;
     const int tj = wall ? 1 : 0;
+    mu = wall ? d.mu[1] : d.mu[0];
     if (d.model == 0) {
-        const double Ys = A.hz_ys[tj], Gs = A.hz_gs[tj], beta = A.hz_beta[tj];
-        double Rs, ms;
-        if (wall) {
-            Rs = rad_i;
-            ms = mass_i;
-            mu = d.mu[1];
-        } else {
-            Rs = 1.0 / (1.0 / rad_i + 1.0 / rad_j);
-            ms = 1.0 / (1.0 / mass_i + 1.0 / mass_j);
-            mu = 0.5 * (d.mu[0] + d.mu[0]);
-        }
-        const double Sn = 2.0 * Ys * sqrt(Rs * delta_n);
-        const double St = 8.0 * Gs * sqrt(Rs * delta_n);
-        const double kn = 4.0 / 3.0 * Ys * sqrt(Rs * delta_n);
-        const double gn = -2.0 * beta * sqrt(5.0 / 6.0 * Sn * ms);
-        kt = 8.0 * Gs * sqrt(Rs * delta_n);
-        gt = -2.0 * beta * sqrt(5.0 / 6.0 * St * ms);
+        const double x = sqrt64(Rs * delta_n), y = sqrt64(x * ms);
+        const double kn = A.hz_kn[tj] * x, gn = A.hz_gn[tj] * y;
+        kt = A.hz_kt[tj] * x;
+        gt = A.hz_gt[tj] * y;
         F0 = -kn * gap - gn * vc[0];
     } else {
-        double kns, kss, dpn, dps, ms;
+        double kns, kss, dpn, dps;
+        dpn = d.dpn[0];
+        dps = d.dps[0];
         if (wall) {
-            kns = d.kn[0]; kss = d.ks[0]; dpn = d.dpn[0]; dps = d.dps[0];
-            ms = mass_i;
-            mu = d.mu[1];
+            kns = d.kn[0]; kss = d.ks[0];
         } else {
-            kns = d.kn[0] * d.kn[0] / (d.kn[0] + d.kn[0]);
-            kss = d.ks[0] * d.ks[0] / (d.ks[0] + d.ks[0]);
-            dpn = 0.5 * (d.dpn[0] + d.dpn[0]);
-            dps = 0.5 * (d.dps[0] + d.dps[0]);
-            ms = 1.0 / (1.0 / mass_i + 1.0 / mass_j);
-            mu = 0.5 * (d.mu[0] + d.mu[0]);
+            kns = 0.5 * d.kn[0]; kss = 0.5 * d.ks[0];   // two equal springs in series
         }
-        const double Cn = 2. * dpn * sqrt(kns * ms);
-        const double Ct = 2. * dps * sqrt(kns * ms);
+        const double c = 2. * sqrt64(kns * ms);
+        const double Cn = dpn * c;
+        const double Ct = dps * c;
         kt = kss;
         gt = Ct;
         F0 = -kns * gap - Cn * vc[0];
     }
     for (int a = 0; a < 3; ++a) shear[a] += inc[a];
     const double ts[3] = {-kt * shear[0], -kt * shear[1], -kt * shear[2]};
-    const double tl = sqrt(dot3(ts, ts));
+    const double tl = sqrt64(dot3(ts, ts));
     F[0] = F0;
     if (tl >= mu * F0 && tl > 0.0) {
-        const double ratio = mu * F0 / tl;
-        F[1] = ts[1] * ratio;
-        F[2] = ts[2] * ratio;
-        shear[1] = -F[1] / kt;
-        shear[2] = -F[2] / kt;
+        // sliding: the spring is set to the friction limit, F = -kt shear
+        const double ratio = mu * F0 * rcp64(tl);
+        shear[1] *= ratio;
+        shear[2] *= ratio;
+        F[1] = -kt * shear[1];
+        F[2] = -kt * shear[2];
     } else {
         F[1] = ts[1] - gt * vc[1];
         F[2] = ts[2] - gt * vc[2];
@@ -214,6 +237,40 @@ __device__ __forceinline__ void periodic_delta(const lbdem_dem &d, const double 
 struct PState {
     double p[3], v[3], w[3], rad, mass;
 };
+
+// The evaluated part of resolve(i, j) (demsolver.py:676-740) for a touching
+// pair, on values in registers: dv is the minimum-image vector i -> j, il the
+// reciprocal of its length, sh the
+// pair's shear history (updated).  Gives the contact point, the force in the
+// contact frame, the lever arms and the force on j (that on i is its exact
+// negative).
+__device__ __forceinline__ void pair_force(const DemArgs &A, const double *pi, const double *vi, const double *wi,
+                                           double rad_i, const double *vj, const double *wj, double Rs, double ms,
+                                           const double *dv, double il, double gap, double *sh, double *cp_out,
+                                           double *F_out, double *ri, double *rj, double *Fj) {
+    const double a[3] = {dv[0] * il, dv[1] * il, dv[2] * il};
+    const M3 R = rot_to_x(a);
+    const double delta_n = -gap;
+    for (int t = 0; t < 3; ++t) {
+        const double cp = pi[t] + a[t] * (rad_i - delta_n);
+        cp_out[t] = cp;
+        ri[t] = cp - pi[t];
+        rj[t] = cp - (pi[t] + dv[t]);
+    }
+    double vci[3], vcj[3], dvc[3], vc[3];
+    cross3(wi, ri, vci);
+    cross3(wj, rj, vcj);
+    for (int t = 0; t < 3; ++t) {
+        vci[t] += vi[t];
+        vcj[t] += vj[t];
+        dvc[t] = vcj[t] - vci[t];
+    }
+    mv(R, dvc, vc);
+    double F[3];
+    contact_force(A, Rs, ms, false, sh, delta_n, vc, F);
+    for (int t = 0; t < 3; ++t) F_out[t] = F[t];
+    mtv(R, F, Fj);
+}
 
 // resolve(i, j) (demsolver.py:638-740); forces on i accumulated in Fi/Mi,
 // forces on j added atomically.  hk: i's first contact slots (the partner of
@@ -244,8 +301,8 @@ __device__ __forceinline__ void resolve_pair(const DemArgs &A, int i, const PSta
             }
     double dv[3];
     periodic_delta(d, P.p, pj, dv);
-    const double distance = sqrt(dot3(dv, dv));
-    const double gap = distance - P.rad - rad_j;
+    const double d2 = dot3(dv, dv), il = rsqrt64(d2);
+    const double gap = sqrt64(d2, il) - P.rad - rad_j;
     bool eval = false;
     if (off >= 0) {
         if (gap < 0) eval = true;
@@ -267,43 +324,15 @@ __device__ __forceinline__ void resolve_pair(const DemArgs &A, int i, const PSta
     if (!eval) return;
     const size_t s = base + off;
     double sh[3] = {d.cf_shear[3 * s], d.cf_shear[3 * s + 1], d.cf_shear[3 * s + 2]};
-    const double len = sqrt(dot3(dv, dv));
-    const double a[3] = {dv[0] / len, dv[1] / len, dv[2] / len};
-    const M3 R = rot_to_x(a);
-    const double delta_n = -gap;
-    const double *pi = P.p;
-    double cp[3], ri[3], rj[3];
-    for (int t = 0; t < 3; ++t) {
-        cp[t] = pi[t] + a[t] * (P.rad - delta_n);
-        d.cf_pos[3 * s + t] = cp[t];
-    }
-    for (int t = 0; t < 3; ++t) {
-        ri[t] = cp[t] - pi[t];
-        rj[t] = cp[t] - (pi[t] + dv[t]);
-    }
-    double vci[3], vcj[3], dvc[3], vc[3];
-    cross3(P.w, ri, vci);
-    cross3(wj, rj, vcj);
-    for (int t = 0; t < 3; ++t) {
-        vci[t] += P.v[t];
-        vcj[t] += vj[t];
-        dvc[t] = vcj[t] - vci[t];
-    }
-    mv(R, dvc, vc);
-    double F[3];
-    contact_force(A, P.rad, P.mass, rad_j, mass_j, false, sh, delta_n, vc, F);
-    for (int t = 0; t < 3; ++t) {
-        d.cf_shear[3 * s + t] = sh[t];
-        d.cf_force[3 * s + t] = F[t];
-    }
-    const M3 Ri = inv3(R);
-    const double mF[3] = {-F[0], -F[1], -F[2]};
-    double Fi[3], Fj[3], Mi[3], Mj[3];
-    mv(Ri, mF, Fi);
-    mv(Ri, F, Fj);
+    double ri[3], rj[3], Fj[3], Mi[3], Mj[3], Rs, ms;
+    pair_effective(P.rad, rad_j, P.mass, mass_j, Rs, ms);
+    pair_force(A, P.p, P.v, P.w, P.rad, vj, wj, Rs, ms, dv, il, gap, sh, d.cf_pos + 3 * s, d.cf_force + 3 * s, ri,
+               rj, Fj);
+    const double Fi[3] = {-Fj[0], -Fj[1], -Fj[2]};
     cross3(ri, Fi, Mi);
     cross3(rj, Fj, Mj);
     for (int t = 0; t < 3; ++t) {
+        d.cf_shear[3 * s + t] = sh[t];
         Fi_acc[t] += Fi[t];
         Mi_acc[t] += Mi[t];
         atomicAdd(d.acc_force + 3 * j + t, Fj[t]);
@@ -311,12 +340,13 @@ __device__ __forceinline__ void resolve_pair(const DemArgs &A, int i, const PSta
     }
 }
 
-// evaluate_wall (demsolver.py:742-807)
-__device__ void wall_contact(const DemArgs &A, int i, const PState &P, int w, double *Fi_acc, double *Mi_acc) {
+// evaluate_wall (demsolver.py:742-807) on values in registers: sh is the wall
+// contact's shear history (updated), cp and F receive the contact point and
+// the force in the contact frame.
+__device__ __forceinline__ void wall_force(const DemArgs &A, const PState &P, int w, double *sh, double *cp, double *F,
+                                           double *Fi_acc, double *Mi_acc) {
     const lbdem_dem &d = A.d;
     const double *nrm = d.wall_n + 3 * w;
-    const size_t s = (size_t)i * 6 + w;
-    double sh[3] = {d.wcf_shear[3 * s], d.wcf_shear[3 * s + 1], d.wcf_shear[3 * s + 2]};
     const M3 R = rot_to_x(nrm);
     const double *p = P.p;
     const double delta_n = (dot3(p, nrm) - d.wall_d[w]) + P.rad;
@@ -324,26 +354,32 @@ __device__ void wall_contact(const DemArgs &A, int i, const PState &P, int w, do
     double ri[3];
     for (int t = 0; t < 3; ++t) {
         ri[t] = distance * nrm[t];
-        d.wcf_pos[3 * s + t] = p[t] + ri[t];
+        cp[t] = p[t] + ri[t];
     }
     double vci[3], m[3], vc[3];
     cross3(P.w, ri, vci);
     for (int t = 0; t < 3; ++t) m[t] = -(vci[t] + P.v[t]);
     mv(R, m, vc);
-    double F[3];
-    contact_force(A, P.rad, P.mass, 0.0, 0.0, true, sh, delta_n, vc, F);
-    for (int t = 0; t < 3; ++t) {
-        d.wcf_shear[3 * s + t] = sh[t];
-        d.wcf_force[3 * s + t] = F[t];
-    }
-    const M3 Ri = inv3(R);
+    contact_force(A, P.rad, P.mass, true, sh, delta_n, vc, F);
     const double mF[3] = {-F[0], -F[1], -F[2]};
     double Fi[3], Mi[3];
-    mv(Ri, mF, Fi);
+    mtv(R, mF, Fi);
     cross3(ri, Fi, Mi);
     for (int t = 0; t < 3; ++t) {
         Fi_acc[t] += Fi[t];
         Mi_acc[t] += Mi[t];
+    }
+}
+
+__device__ void wall_contact(const DemArgs &A, int i, const PState &P, int w, double *Fi_acc, double *Mi_acc) {
+    const lbdem_dem &d = A.d;
+    const size_t s = (size_t)i * 6 + w;
+    double sh[3] = {d.wcf_shear[3 * s], d.wcf_shear[3 * s + 1], d.wcf_shear[3 * s + 2]}, cp[3], F[3];
+    wall_force(A, P, w, sh, cp, F, Fi_acc, Mi_acc);
+    for (int t = 0; t < 3; ++t) {
+        d.wcf_pos[3 * s + t] = cp[t];
+        d.wcf_shear[3 * s + t] = sh[t];
+        d.wcf_force[3 * s + t] = F[t];
     }
 }
 
@@ -495,15 +531,22 @@ __device__ M3 quat2rot(const double *q) {
     return r;
 }
 
-// Euler rotation update (demsolver.py:590-636) on values already in registers:
-// q (4), w (3), wd (3, previous angular acceleration), moment (3), inertia (9).
-__device__ void rotate_update(double dt, double q[4], double w[3], double wd[3], const double mom[3],
-                              const double inertia[9]) {
+// Angular acceleration (demsolver.py:590-613) R^-1 I^-1 (R M - (R w) x I (R w)).
+// For a multiple of the unit tensor -- every sphere -- it is M / I whatever the
+// orientation, which takes the quaternion and eight dependent products out of
+// a sub-step's chain; other tensors (the field is the user's) take the general
+// form.
+__device__ __forceinline__ bool inertia_iso(const double I[9]) {
+    return I[0] == I[4] && I[0] == I[8] && I[1] == 0.0 && I[2] == 0.0 && I[3] == 0.0 && I[5] == 0.0 && I[6] == 0.0 &&
+           I[7] == 0.0;
+}
+__device__ __noinline__ void angular_general(const double *q, const double *w, const double *mom, const double *inertia,
+                                             double *alpha) {
     const M3 Rm = quat2rot(q);
     M3 I;
     for (int r = 0; r < 3; ++r)
         for (int c = 0; c < 3; ++c) I.m[r][c] = inertia[3 * r + c];
-    double ml[3], wl[3], Iw[3], cw[3], rhs[3], wdl[3], alpha[3];
+    double ml[3], wl[3], Iw[3], cw[3], rhs[3], wdl[3];
     mv(Rm, mom, ml);
     mv(Rm, w, wl);
     mv(I, wl, Iw);
@@ -511,15 +554,22 @@ __device__ void rotate_update(double dt, double q[4], double w[3], double wd[3],
     for (int t = 0; t < 3; ++t) rhs[t] = ml[t] - cw[t];
     mv(inv3(I), rhs, wdl);
     mv(inv3(Rm), wdl, alpha);
+}
+
+// Euler rotation update (demsolver.py:614-636) on values already in registers:
+// w (3), wd (3, the previous angular acceleration) and the new one; q (4).
+__device__ __forceinline__ void spin_update(double dt, double w[3], double wd[3], const double alpha[3]) {
     for (int t = 0; t < 3; ++t) w[t] += 0.5 * (wd[t] + alpha[t]) * dt;
+    for (int t = 0; t < 3; ++t) wd[t] = alpha[t];
+}
+__device__ __forceinline__ void quat_update(double dt, double q[4], const double w[3]) {
     const double dq0 = -0.5 * (q[1] * w[0] + q[2] * w[1] + q[3] * w[2]);
     const double dq1 = +0.5 * (q[0] * w[0] - q[3] * w[1] + q[2] * w[2]);
     const double dq2 = +0.5 * (q[3] * w[0] + q[0] * w[1] + q[1] * w[2]);
     const double dq3 = +0.5 * (-q[2] * w[0] + q[1] * w[1] + q[0] * w[2]);
     q[0] += dq0 * dt; q[1] += dq1 * dt; q[2] += dq2 * dt; q[3] += dq3 * dt;
-    const double ql = sqrt(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
-    for (int t = 0; t < 4; ++t) q[t] = q[t] / ql;
-    for (int t = 0; t < 3; ++t) wd[t] = alpha[t];
+    const double il = rsqrt64((q[0] * q[0] + q[1] * q[1]) + (q[2] * q[2] + q[3] * q[3]));
+    for (int t = 0; t < 4; ++t) q[t] *= il;
 }
 
 __device__ __forceinline__ void wrap_position(const lbdem_dem &d, double *p) {
@@ -532,6 +582,21 @@ __device__ __forceinline__ void wrap_position(const lbdem_dem &d, double *p) {
     }
 }
 
+// update (demsolver.py:514-589), translation on values in registers; the
+// position is not wrapped yet.
+__device__ __forceinline__ void translate_update(double dt, int fixed, double imass, const double force[3], double p[3],
+                                                 double v[3], double acc[3]) {
+    if (fixed) {
+        for (int t = 0; t < 3; ++t) p[t] += v[t] * dt;
+        return;
+    }
+    double a[3];
+    for (int t = 0; t < 3; ++t) a[t] = force[t] * imass;
+    for (int t = 0; t < 3; ++t) v[t] += 0.5 * (acc[t] + a[t]) * dt;
+    for (int t = 0; t < 3; ++t) p[t] += v[t] * dt + 0.5 * a[t] * (dt * dt);
+    for (int t = 0; t < 3; ++t) acc[t] = a[t];
+}
+
 __device__ void integrate_particle(const lbdem_dem &d, int ncell, int parity, int i, int role);
 __device__ __forceinline__ void integrate_unit(const lbdem_dem &d, int ncell, int parity, int u);
 
@@ -542,6 +607,38 @@ __global__ void __launch_bounds__(128) k_integrate(const __grid_constant__ DemAr
     int32_t *used = d.cell_count + (size_t)A.parity * A.ncell;
     for (int c = tid; c < A.ncell; c += gridDim.x * blockDim.x) used[c] = 0;
     if (tid < 3 * d.n) integrate_unit(d, A.ncell, A.parity, tid);
+}
+
+// late_clear_state / remove_inactive_contact (demsolver.py:371-386, 431-436):
+// slots are only moved when an inactive one precedes an active one.  Returns
+// the number of active slots among the first `used`.
+__device__ __forceinline__ int compact_slots(const lbdem_dem &d, int i, int used) {
+    const size_t base = (size_t)i * d.maxc;
+    int act[SLOTS_IN_REGS];
+#pragma unroll
+    for (int o = 0; o < SLOTS_IN_REGS; ++o) act[o] = o < d.maxc ? d.cf_active[base + o] : 0;
+    const int cnt = min(used, d.maxc);
+    int w_ = 0;
+    auto keep = [&](int o) {
+        if (w_ != o) {
+            const size_t dd = base + w_, ss = base + o;
+            d.cf_j[dd] = d.cf_j[ss];
+            d.cf_active[dd] = 1;
+            for (int t = 0; t < 3; ++t) {
+                d.cf_shear[3 * dd + t] = d.cf_shear[3 * ss + t];
+                d.cf_pos[3 * dd + t] = d.cf_pos[3 * ss + t];
+                d.cf_force[3 * dd + t] = d.cf_force[3 * ss + t];
+            }
+        }
+        ++w_;
+    };
+#pragma unroll
+    for (int o = 0; o < SLOTS_IN_REGS; ++o)
+        if (o < cnt && act[o]) keep(o);
+    for (int o = SLOTS_IN_REGS; o < cnt; ++o)
+        if (d.cf_active[base + o]) keep(o);
+    for (int o = w_; o < cnt; ++o) d.cf_active[base + o] = 0;
+    return w_;
 }
 
 __device__ void integrate_particle(const lbdem_dem &d, int ncell, int parity, int i, int role) {
@@ -568,17 +665,8 @@ __device__ void integrate_particle(const lbdem_dem &d, int ncell, int parity, in
             force[t] = f;
         }
         if (!frozen) {
-            if (fixed) {
-                for (int t = 0; t < 3; ++t) p[t] += v[t] * dt;
-                wrap_position(d, p);
-            } else {
-                double a[3];
-                for (int t = 0; t < 3; ++t) a[t] = force[t] / mass;
-                for (int t = 0; t < 3; ++t) v[t] += 0.5 * (acc[t] + a[t]) * dt;
-                for (int t = 0; t < 3; ++t) p[t] += v[t] * dt + 0.5 * a[t] * (dt * dt);
-                wrap_position(d, p);
-                for (int t = 0; t < 3; ++t) acc[t] = a[t];
-            }
+            translate_update(dt, fixed, rcp64(mass), force, p, v, acc);
+            wrap_position(d, p);
         }
         for (int t = 0; t < 3; ++t) {
             d.acc_force[3 * i + t] = 0.0;
@@ -617,7 +705,17 @@ __device__ void integrate_particle(const lbdem_dem &d, int ncell, int parity, in
             m += mfl[t];
             moment[t] = m;
         }
-        if (!frozen) rotate_update(dt, q, w, wd, moment, I);
+        if (!frozen) {
+            double alpha[3];
+            if (inertia_iso(I)) {
+                const double iI = rcp64(I[0]);
+                for (int t = 0; t < 3; ++t) alpha[t] = moment[t] * iI;
+            } else {
+                angular_general(q, w, moment, I, alpha);
+            }
+            spin_update(dt, w, wd, alpha);
+            quat_update(dt, q, w);
+        }
         for (int t = 0; t < 3; ++t) {
             d.acc_moment[3 * i + t] = 0.0;
             d.moment[3 * i + t] = moment[t];
@@ -626,34 +724,7 @@ __device__ void integrate_particle(const lbdem_dem &d, int ncell, int parity, in
         }
         for (int t = 0; t < 4; ++t) d.quat[4 * i + t] = q[t];
     } else {
-        // late_clear_state / remove_inactive_contact (demsolver.py:371-386, 431-436):
-        // slots are only moved when an inactive one precedes an active one
-        const size_t base = (size_t)i * d.maxc;
-        const int nfirst = d.cfn[i], nadd = d.cf_add[i];
-        int act[SLOTS_IN_REGS];
-#pragma unroll
-        for (int o = 0; o < SLOTS_IN_REGS; ++o) act[o] = o < d.maxc ? d.cf_active[base + o] : 0;
-        const int cnt = min(nfirst + nadd, d.maxc);
-        int w_ = 0;
-        auto keep = [&](int o) {
-            if (w_ != o) {
-                const size_t dd = base + w_, ss = base + o;
-                d.cf_j[dd] = d.cf_j[ss];
-                d.cf_active[dd] = 1;
-                for (int t = 0; t < 3; ++t) {
-                    d.cf_shear[3 * dd + t] = d.cf_shear[3 * ss + t];
-                    d.cf_pos[3 * dd + t] = d.cf_pos[3 * ss + t];
-                    d.cf_force[3 * dd + t] = d.cf_force[3 * ss + t];
-                }
-            }
-            ++w_;
-        };
-#pragma unroll
-        for (int o = 0; o < SLOTS_IN_REGS; ++o)
-            if (o < cnt && act[o]) keep(o);
-        for (int o = SLOTS_IN_REGS; o < cnt; ++o)
-            if (d.cf_active[base + o]) keep(o);
-        for (int o = w_; o < cnt; ++o) d.cf_active[base + o] = 0;
+        const int w_ = compact_slots(d, i, d.cfn[i] + d.cf_add[i]);
         d.cfn[i] = w_;
         d.cf_add[i] = 0;
     }
@@ -741,11 +812,9 @@ __device__ __forceinline__ void red_release_gpu(unsigned *p, unsigned v) {
 // reduction per block and barrier (after the block barrier, which orders the
 // block's writes of the phase before thread 0, so the release publishes them
 // all), then polling with acquire loads; no reset.
-__device__ __forceinline__ void grid_barrier(uint32_t *sync, unsigned &gen, int32_t *status) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned target = (gen + 1) * gridDim.x;
-        red_release_gpu(sync, 1u);
+__device__ __forceinline__ void grid_wait(uint32_t *sync, unsigned gen, int32_t *status) {
+    if (gridDim.x > 1 && threadIdx.x == 0) {
+        const unsigned target = gen * gridDim.x;
         unsigned it = 0;
         while (ld_acquire_gpu(sync) < target) {
             if (++it > (1u << 22)) {
@@ -755,8 +824,23 @@ __device__ __forceinline__ void grid_barrier(uint32_t *sync, unsigned &gen, int3
             __nanosleep(32);
         }
     }
-    gen += 1;
     __syncthreads();
+}
+__device__ __forceinline__ void grid_barrier(uint32_t *sync, unsigned &gen, int32_t *status) {
+    __syncthreads();
+    if (gridDim.x > 1 && threadIdx.x == 0) red_release_gpu(sync, 1u);
+    gen += 1;
+    grid_wait(sync, gen, status);
+}
+
+// The last block to leave a launch that used grid_barrier resets its counter
+// (sync[1] counts the blocks past their last barrier); true in that thread.
+__device__ __forceinline__ bool barrier_release(uint32_t *sync) {
+    __syncthreads();
+    if (threadIdx.x != 0 || atomicAdd(sync + 1, 1u) != gridDim.x - 1) return false;
+    sync[0] = 0u;
+    sync[1] = 0u;
+    return true;
 }
 
 template <bool WRAP>
@@ -776,20 +860,664 @@ __global__ void __launch_bounds__(128, 1) k_dem_coop(const __grid_constant__ Dem
         for (int u = me; u < 3 * d.n; u += nthr) integrate_unit(d, A.ncell, parity, u);
         grid_barrier(d.sync, gen, d.status);
     }
+    barrier_release(d.sync);
 }
 
-// The per-material Hertz constants of DemArgs, in the operation order of
+// ---------------------------------------------------------------------------
+// All sub-steps of one call in ONE launch without a grid barrier per sub-step:
+// LPP lanes own a particle for the whole call, its state stays in registers,
+// and a particle waits only for the particles it can touch.
+//
+// What bounds the sub-steps is latency: two grid barriers and a chain of
+// dependent loads (cell, list, partner, contact slot) per sub-step, for a few
+// thousand threads.  But a particle moves a fraction of its radius per call,
+// so the pairs that can touch during a chunk of sub-steps are known at its
+// start, and most particles of a suspension have none.  Per chunk:
+//   build   every particle's partners: gap <= m_i + m_j, m the displacement
+//           that its velocity and known acceleration allow (times two) plus
+//           FLOW_SLACK radii.  The test is symmetric bit for bit, so both sides
+//           list the pair.  Shear histories of known contacts are copied to
+//           registers on BOTH sides.
+//   flow    a lane evaluates its pairs from the lower index's perspective (the
+//           same arithmetic on the same values on both sides, so both copies of
+//           the history agree) and keeps its own side's force: no atomics.
+//           A particle with partners publishes its state after a sub-step as
+//           nine 16-byte packets (value, sub-step) in one of two slots; a
+//           partner polls those packets, which is wait and transfer in one
+//           round trip.  Partners are at most one sub-step apart (each needs
+//           the other's state), so two slots suffice.  A warp publishes before
+//           it polls, and every warp is resident, so every wait ends; they are
+//           bounded all the same.
+//   commit  after a grid barrier: state, contact slots and broad-phase lists.
+// Nothing is written before the commit, so a chunk whose assumptions fail -- a
+// particle moved farther than m, more than FLOW_NBR partners, a full contact
+// list, a particle leaving the grid -- is done by the two-phase form instead,
+// in the same launch.
+// 10 sub-steps, against the two-phase form (B200): 2000 spheres of a 256^3
+// suspension, a fifth of them in contact, 45 us (106); one sphere 16 us (60);
+// others at flow_forms.  What bounds it now: FP64 latency of an isolated
+// particle's sub-step 0.65 us, of one with a contact 1.9 us (half of it the
+// exchange through L2), and 12 us of search, barrier and commit per call.
+// ---------------------------------------------------------------------------
+constexpr int FLOW_THREADS = 128;
+constexpr int FLOW_NBR = 16;          // partners of a particle
+constexpr int FLOW_CHUNK = 16;        // sub-steps between two partner searches
+constexpr double FLOW_SLACK = 0.02;   // radii
+// In more than one block, fewer sub-steps than this run the two-phase form: a
+// partner search and commit cost 12-20 us (2000 / 10,000 particles: 29 / 46 us
+// for one sub-step against 18 / 21, 29 / 48 for two against 26 / 40, 31 / 50
+// for three against 35 / 59).
+constexpr int FLOW_MIN_SUBSTEPS = 3;
+constexpr size_t FLOW_HEADER = 256;   // workspace: two failure words (by chunk parity), the epoch, then the packets
+constexpr int FLOW_STRIDE = 16;       // packets between two slots: no 128-byte line is polled and written for two
+constexpr int FLOW_STATE = 9;         // doubles of a published state: position, velocity, angular velocity
+constexpr int FLOW_TAGS = 2 * FLOW_CHUNK;   // tags of a chunk: no packet of an earlier chunk or call has one of them
+
+struct FlowArgs {
+    DemArgs A;
+    unsigned char *work;
+    int nsub;
+};
+
+__device__ __forceinline__ ulonglong2 *flow_packets(const FlowArgs &f, int i, int slot) {
+    return reinterpret_cast<ulonglong2 *>(f.work + FLOW_HEADER) + ((size_t)i * 2 + slot) * FLOW_STRIDE;
+}
+// a packet is one 128-bit relaxed access: value and tag arrive together
+__device__ __forceinline__ void packet_store(bool on, ulonglong2 *p, double v, unsigned long long tag) {
+    const unsigned __int128 w = ((unsigned __int128)tag << 64) | (unsigned long long)__double_as_longlong(v);
+    asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q st.relaxed.gpu.global.b128 [%0], %1;\n}\n" ::"l"(p),
+                 "q"(w), "r"((unsigned)on)
+                 : "memory");
+}
+__device__ __forceinline__ void packet_load(const ulonglong2 *p, unsigned long long &v, unsigned long long &tag) {
+    unsigned __int128 w;
+    asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];" : "=q"(w) : "l"(p) : "memory");
+    v = (unsigned long long)w;
+    tag = (unsigned long long)(w >> 64);
+}
+// one look at a partner's packets: true when all are of sub-step `tag`
+__device__ __forceinline__ bool flow_look(const ulonglong2 *p, unsigned long long tag, double o[FLOW_STATE]) {
+    bool ok = true;
+#pragma unroll
+    for (int c = 0; c < FLOW_STATE; ++c) {
+        unsigned long long v, t;
+        packet_load(p + c, v, t);
+        ok = ok && t == tag;
+        o[c] = __longlong_as_double((long long)v);
+    }
+    return ok;
+}
+
+// Displacement allowed to particle i during T: twice that of its velocity and
+// of the body and fluid force, plus the slack that contacts may use.
+__device__ __forceinline__ double flow_budget(const lbdem_dem &d, int i, double T, double rad, double mass) {
+    // sums of magnitudes, in FP32: a bound needs no more, and FP32 divides in a few cycles
+    float v = 0.f, a = 0.f, g = 0.f;
+    for (int t = 0; t < 3; ++t) {
+        v += fabsf((float)d.vel[3 * i + t]);
+        a += fabsf((float)d.force_fluid[3 * i + t]);
+        g += fabsf((float)d.g[t]);
+    }
+    const float Tf = (float)T;
+    return (double)(2.f * Tf * (v + Tf * (a / (float)mass + g))) + FLOW_SLACK * rad;
+}
+
+// minimum-image vector pi -> pj (periodic_delta) and which periods it took:
+// bits 2a (minus) and 2a + 1 (plus) of axis a
+__device__ __forceinline__ int image_delta(const lbdem_dem &d, const double *pi, const double *pj, double *dv) {
+    int m = 0;
+    for (int a = 0; a < 3; ++a) {
+        dv[a] = pj[a] - pi[a];
+        if (d.periodic[a]) {
+            const double L = d.dom_max[a] - d.dom_min[a];
+            if (dv[a] > 0.5 * L) { dv[a] -= L; m |= 1 << (2 * a); }
+            else if (dv[a] < -0.5 * L) { dv[a] += L; m |= 2 << (2 * a); }
+        }
+    }
+    return m;
+}
+
+// Whether the broad phase proposes the pair (i, j), i the lower index: j's
+// cell among i's own and its octant's (bpcd.py:133-142), or, with periodic
+// images, those of i's images (contact_lane).
+template <bool WRAP>
+__device__ __noinline__ bool flow_proposed(const lbdem_dem &d, double px, double py, double pz, double ox, double oy,
+                                           double oz) {
+    const double pi[3] = {px, py, pz}, pj[3] = {ox, oy, oz};
+    int cj[3];
+    ref_cell(d, pj, cj);
+    double sh[3] = {0.0, 0.0, 0.0};
+    if (WRAP)
+        for (int a = 0; a < 3; ++a) {
+            if (!d.periodic[a]) continue;
+            const double L = d.dom_max[a] - d.dom_min[a];
+            if (pi[a] < d.dom_min[a] + d.cell_size) sh[a] = L;
+            else if (pi[a] > d.dom_max[a] - d.cell_size) sh[a] = -L;
+        }
+    for (int im = 0; im < (WRAP ? 8 : 1); ++im) {
+        bool in = true;
+        for (int a = 0; a < 3; ++a) {
+            const bool img = (im >> a) & 1;
+            if (img && sh[a] == 0.0) in = false;
+            const double q = pi[a] + (img ? sh[a] : 0.0);
+            const int c = (int)floor((q - d.bp_min[a]) / d.cell_size);
+            const double center = (c + 0.5) * d.cell_size + d.bp_min[a];
+            const int o = cj[a] - c;
+            in = in && (o == 0 || o == (q > center ? 1 : -1));
+        }
+        if (in) return true;
+    }
+    return false;
+}
+
+// the two-phase form over the sub-steps of a chunk whose lists are binned in
+// half `parity` (the body of k_dem_coop)
+template <bool WRAP>
+__device__ __noinline__ void flow_two_phase(const DemArgs &A, int parity, int nsub, unsigned &gen) {
+    const lbdem_dem &d = A.d;
+    const int nthr = gridDim.x * blockDim.x, me = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int s = 0; s < nsub; ++s) {
+        const int par = (parity + s) & 1;
+        int32_t *count = d.cell_count + (size_t)par * A.ncell;
+        for (int base = 0; base < 8 * d.n; base += nthr) contact_lane<WRAP>(A, count, base + me);
+        grid_barrier(d.sync, gen, d.status);
+        for (int c = me; c < A.ncell; c += nthr) count[c] = 0;
+        for (int u = me; u < 3 * d.n; u += nthr) integrate_unit(d, A.ncell, par, u);
+        grid_barrier(d.sync, gen, d.status);
+    }
+}
+
+// MB: resident blocks per SM the registers are cut for (2: none spilled; 3: 168 registers, some spills)
+template <bool WRAP, int LPP, int MB>
+__global__ void __launch_bounds__(FLOW_THREADS, MB) k_dem_flow(const __grid_constant__ FlowArgs f) {
+    constexpr int GPB = FLOW_THREADS / LPP;          // particles per block
+    constexpr int K = FLOW_NBR / LPP;                // pairs per lane
+    constexpr int NW = (6 + LPP - 1) / LPP;          // walls per lane
+    __shared__ int s_cnt[GPB], s_list[GPB][FLOW_NBR];
+    __shared__ double s_I[GPB][9];                   // inertia tensors
+    const DemArgs &A = f.A;
+    const lbdem_dem &d = A.d;
+    const int nthr = gridDim.x * blockDim.x, me = blockIdx.x * blockDim.x + threadIdx.x;
+    const int g = threadIdx.x / LPP, k = threadIdx.x % LPP;
+    const int i = blockIdx.x * GPB + g;
+    const bool act = i < d.n;
+    const double rmax = 0.25 * d.cell_size;
+    int *fail_words = reinterpret_cast<int *>(f.work);
+    unsigned long long *epoch = reinterpret_cast<unsigned long long *>(f.work + 16);
+    const unsigned long long epoch0 = *epoch;
+    unsigned gen = 0;
+    int parity = A.parity, done = 0, chunk = 0;
+    while (done < f.nsub) {
+        const int S = min(f.nsub - done, FLOW_CHUNK);
+        const unsigned long long tag0 = epoch0 + (unsigned long long)chunk * FLOW_TAGS;
+        volatile int *fail = fail_words + (chunk & 1);
+        int32_t *count = d.cell_count + (size_t)parity * A.ncell;
+        // ------------------------------------------------------------ build
+        PState P = {};
+        double acc[3] = {}, wd[3] = {}, q[4] = {}, ffl[3] = {}, mfl[3] = {}, af[3] = {}, am[3] = {};
+        double m = 0.0, imass = 0.0, iI = 0.0;
+        int frozen = 1, fixed = 0, n_used = 0;
+        bool bad = false, iso = true;
+        if (k == 0) s_cnt[g] = 0;
+        __syncwarp();
+        if (act) {
+            for (int t = 0; t < 3; ++t) {
+                P.p[t] = d.pos[3 * i + t];
+                P.v[t] = d.vel[3 * i + t];
+                P.w[t] = d.omega[3 * i + t];
+                acc[t] = d.acc[3 * i + t];
+                wd[t] = d.omega_dot[3 * i + t];
+                ffl[t] = d.force_fluid[3 * i + t];
+                mfl[t] = d.moment_fluid[3 * i + t];
+                af[t] = d.acc_force[3 * i + t];
+                am[t] = d.acc_moment[3 * i + t];
+            }
+            for (int t = 0; t < 4; ++t) q[t] = d.quat[4 * i + t];
+            P.rad = d.radius[i];
+            P.mass = d.mass[i];
+            frozen = d.freeze[i];
+            fixed = d.fixvel[i];
+            n_used = d.cfn[i];
+            double I[9];
+            for (int t = 0; t < 9; ++t) I[t] = d.inertia[9 * i + t];
+            iso = inertia_iso(I);
+            iI = rcp64(I[0]);
+            imass = rcp64(P.mass);
+            if (!iso && k == 0)
+                for (int t = 0; t < 9; ++t) s_I[g][t] = I[t];
+            const double T = S * d.dt, mcap = 0.25 * rmax;
+            m = flow_budget(d, i, T, P.rad, P.mass);
+            bad = !(m <= mcap);
+            // cells that hold every possible partner: centres within reach, of
+            // the particle and of its periodic images
+            const double reach = P.rad + rmax + m + mcap;
+            // (a superset: a reciprocal and a slack do).  Per axis: n0 cells of
+            // the particle from lo0, then n1 of its image from lo1
+            const double icell = rcp64(d.cell_size);
+            int lo0[3], lo1[3], n0[3], n1[3], code[3];
+            for (int a = 0; a < 3; ++a) {
+                const double x = P.p[a] - d.bp_min[a];
+                bad = bad || !(x - m > -d.cell_size && x + m < (d.gdim[a] - 1) * d.cell_size);
+                lo0[a] = max(-1, (int)floor((x - reach) * icell - 1e-9));
+                n0[a] = max(0, min(d.gdim[a] - 2, (int)floor((x + reach) * icell + 1e-9)) - lo0[a] + 1);
+                lo1[a] = n1[a] = code[a] = 0;
+                if (!d.periodic[a]) continue;
+                const double L = d.dom_max[a] - d.dom_min[a];
+                double sh = 0.0;
+                if (P.p[a] < d.dom_min[a] + reach) { sh = L; code[a] = 1 << (2 * a); }
+                else if (P.p[a] > d.dom_max[a] - reach) { sh = -L; code[a] = 2 << (2 * a); }
+                if (sh != 0.0) {
+                    lo1[a] = max(-1, (int)floor((x + sh - reach) * icell - 1e-9));
+                    n1[a] = max(0, min(d.gdim[a] - 2, (int)floor((x + sh + reach) * icell + 1e-9)) - lo1[a] + 1);
+                }
+            }
+            const int nx = n0[0] + n1[0], nxy = nx * (n0[1] + n1[1]), tot = bad ? 0 : nxy * (n0[2] + n1[2]);
+            const float inx = 1.f / (float)nx, inxy = 1.f / (float)nxy;
+            auto consider = [&](int j, const double *pj, double rj, int image) {
+                double dv[3];
+                if (image_delta(d, P.p, pj, dv) != image) return;        // found through another image
+                const double d2 = dot3(dv, dv), far = P.rad + rj + (m + mcap);
+                if (!(d2 <= far * far)) return;
+                const double near = P.rad + rj + (m + flow_budget(d, j, T, rj, d.mass[j]));
+                if (!(d2 <= near * near)) return;
+                const int at = atomicAdd(&s_cnt[g], 1);
+                if (at < FLOW_NBR) s_list[g][at] = j;
+                else bad = true;
+            };
+            for (int c0 = k; c0 < tot; c0 += 2 * LPP) {
+                // two cells at a time: counts and first two entries in one round
+                // trip, those particles' positions in a second
+                int ci[2], nj[2], image[2], e[2][2];
+                double pj[2][2][3], rj[2][2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int c = c0 + u * LPP;
+                    ci[u] = image[u] = nj[u] = e[u][0] = e[u][1] = 0;
+                    if (c >= tot) continue;
+                    const int iz = (int)(((float)c + 0.5f) * inxy), r = c - iz * nxy;
+                    const int iy = (int)(((float)r + 0.5f) * inx), ix = r - iy * nx;
+                    const bool bx = ix >= n0[0], by = iy >= n0[1], bz = iz >= n0[2];
+                    image[u] = (bx ? code[0] : 0) | (by ? code[1] : 0) | (bz ? code[2] : 0);
+                    ci[u] = cell_index(d, bx ? lo1[0] + ix - n0[0] : lo0[0] + ix, by ? lo1[1] + iy - n0[1] : lo0[1] + iy,
+                                       bz ? lo1[2] + iz - n0[2] : lo0[2] + iz);
+                    const int32_t *lst = d.cell_list + (size_t)ci[u] * d.cell_cap;
+                    nj[u] = count[ci[u]];
+                    e[u][0] = lst[0];
+                    e[u][1] = d.cell_cap > 1 ? lst[1] : 0;
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    bad = bad || nj[u] > d.cell_cap;
+                    nj[u] = min(nj[u], d.cell_cap);
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) {
+                        if (t >= nj[u]) e[u][t] = i;
+                        const int j = e[u][t];
+                        for (int a = 0; a < 3; ++a) pj[u][t][a] = d.pos[3 * j + a];
+                        rj[u][t] = d.radius[j];
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+#pragma unroll
+                    for (int t = 0; t < 2; ++t)
+                        if (e[u][t] != i) consider(e[u][t], pj[u][t], rj[u][t], image[u]);
+                    for (int t = 2; t < nj[u]; ++t) {
+                        const int j = d.cell_list[(size_t)ci[u] * d.cell_cap + t];
+                        const double p[3] = {d.pos[3 * j], d.pos[3 * j + 1], d.pos[3 * j + 2]};
+                        if (j != i) consider(j, p, d.radius[j], image[u]);
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        // this lane's pairs: partner, its constants, and the shear history of a
+        // contact that the lower index already lists
+        const int nn = act ? min(s_cnt[g], FLOW_NBR) : 0;
+        int pj[K], pslot[K];                       // partner; slot of the lower index, -1: none yet
+        unsigned pact = 0, pdirty = 0;             // bit e: pair e is in contact / was evaluated
+        double prad[K], pRs[K], pms[K], psh[K][3], pcp[K][3], pF[K][3];
+        int np = 0, matched = 0;
+        for (int e = k; e < nn; e += LPP, ++np) {
+            const int j = s_list[g][e], own = min(i, j), other = max(i, j);
+            pj[np] = j;
+            prad[np] = d.radius[j];
+            pair_effective(P.rad, prad[np], P.mass, d.mass[j], pRs[np], pms[np]);
+            const int no = min(d.cfn[own], d.maxc);
+            int off = -1;
+            for (int o = 0; o < no && off < 0; ++o)
+                if (d.cf_j[(size_t)own * d.maxc + o] == other && d.cf_active[(size_t)own * d.maxc + o]) off = o;
+            pslot[np] = off;
+            for (int t = 0; t < 3; ++t) psh[np][t] = off >= 0 ? d.cf_shear[3 * ((size_t)own * d.maxc + off) + t] : 0.0;
+            if (off >= 0) {
+                pact |= 1u << np;
+                matched += own == i;
+            }
+        }
+        __syncwarp();
+        for (int o = 1; o < LPP; o <<= 1) matched += __shfl_xor_sync(0xffffffffu, matched, o);
+        const int np_most = __reduce_max_sync(0xffffffffu, np);
+        const int room = d.maxc - (n_used - matched);     // slots for listed pairs
+        int wact = 0, wdirty = 0, wnear = 0;
+        double wsh[NW][3], wcp[NW][3], wF[NW][3];
+        for (int e = 0; e < NW; ++e) {
+            const int w = k + e * LPP;
+            if (!act || w >= 6 || d.wall_periodic[w]) continue;
+            if (d.wcf_active[(size_t)i * 6 + w]) wact |= 1 << e;
+            // walls within the particle's displacement (normals are unit vectors; any other length only widens it)
+            const double *nrm = d.wall_n + 3 * w;
+            const double sep = -(dot3(P.p, nrm) - d.wall_d[w]);
+            if (((wact >> e) & 1) || !(sep > P.rad + m * (fabs(nrm[0]) + fabs(nrm[1]) + fabs(nrm[2])))) wnear |= 1 << e;
+            for (int t = 0; t < 3; ++t) wsh[e][t] = d.wcf_shear[3 * ((size_t)i * 6 + w) + t];
+        }
+        if (bad) *fail = 1;
+        // half a grid barrier: the lists may be cleared once every block has built
+        __syncthreads();
+        if (threadIdx.x == 0 && gridDim.x > 1) red_release_gpu(d.sync, 1u);
+        ++gen;
+        bool failed;
+        {
+            // -------------------------------------------------------- flow
+            double D[3] = {0.0, 0.0, 0.0}, force[3], moment[3];
+            bool lost = false, late = false;
+            const bool walls = __any_sync(0xffffffffu, wnear != 0);
+            for (int s = 0; s < S; ++s) {
+                double F[3] = {0.0, 0.0, 0.0}, M[3] = {0.0, 0.0, 0.0};
+                int held = 0, fresh = 0;
+                bool hit = false;                         // this lane evaluated a contact
+                for (int e = 0; e < np_most; ++e) {
+                    const bool have = e < np;
+                    const int j = have ? pj[e] : i;
+                    const bool own = i < j;
+                    double o[FLOW_STATE];
+                    if (s == 0) {
+                        if (have)
+                            for (int t = 0; t < 3; ++t) {
+                                o[t] = d.pos[3 * j + t];
+                                o[3 + t] = d.vel[3 * j + t];
+                                o[6 + t] = d.omega[3 * j + t];
+                            }
+                    } else {
+                        // The warp polls as one: a lane spinning by itself leaves the warp split, and every
+                        // later exchange between its lanes then costs hundreds of cycles (a contact between
+                        // two SMs: 14,300 cycles per sub-step with a loop per lane).  Bounded: about 2^20 looks.
+                        bool wait = have && !lost;
+                        for (unsigned it = 0; __any_sync(0xffffffffu, wait); ++it) {
+                            if (wait) {
+                                const int failed = *fail;
+                                wait = !flow_look(flow_packets(f, j, s & 1), tag0 + s, o);
+                                if (wait && (failed || it >= (1u << 20))) {
+                                    late = late || !failed;
+                                    lost = true;          // the chunk has failed: no more waits
+                                    wait = false;
+                                }
+                            }
+                        }
+                    }
+                    if (have && !lost) {
+                        double lp[3], hp[3], dv[3];
+                        for (int t = 0; t < 3; ++t) {
+                            lp[t] = own ? P.p[t] : o[t];
+                            hp[t] = own ? o[t] : P.p[t];
+                        }
+                        const int img = image_delta(d, lp, hp, dv);
+                        const bool on = (pact >> e) & 1u;
+                        held += own && on;
+                        const double lr = own ? P.rad : prad[e], hr = own ? prad[e] : P.rad;
+                        const double d2 = dot3(dv, dv), il = rsqrt64(d2), gap = sqrt64(d2, il) - lr - hr;
+                        // (the reference proposes no pair across a periodic face)
+                        const bool proposed = WRAP || img == 0;
+                        if (proposed && !(gap < 0) && on &&
+                            flow_proposed<WRAP>(d, lp[0], lp[1], lp[2], hp[0], hp[1], hp[2]))
+                            pact &= ~(1u << e);
+                        if (proposed && gap < 0) {
+                            double lv[3], lw[3], hv[3], hw[3], shr[3], cp[3], Fc[3], ri[3], rj[3], Fj[3], Ms[3];
+                            for (int t = 0; t < 3; ++t) {
+                                lv[t] = own ? P.v[t] : o[3 + t];
+                                lw[t] = own ? P.w[t] : o[6 + t];
+                                hv[t] = own ? o[3 + t] : P.v[t];
+                                hw[t] = own ? o[6 + t] : P.w[t];
+                                shr[t] = on ? psh[e][t] : 0.0;
+                            }
+                            fresh += own && !on;
+                            pact |= 1u << e;
+                            pdirty |= 1u << e;
+                            pair_force(A, lp, lv, lw, lr, hv, hw, pRs[e], pms[e], dv, il, gap, shr, cp, Fc, ri, rj, Fj);
+                            hit = true;
+                            for (int t = 0; t < 3; ++t) {
+                                psh[e][t] = shr[t];
+                                pcp[e][t] = cp[t];
+                                pF[e][t] = Fc[t];
+                                ri[t] = own ? ri[t] : rj[t];
+                                Fj[t] = own ? -Fj[t] : Fj[t];
+                            }
+                            cross3(ri, Fj, Ms);
+                            for (int t = 0; t < 3; ++t) {
+                                F[t] += Fj[t];
+                                M[t] += Ms[t];
+                            }
+                        }
+                    }
+                    __syncwarp();
+                }
+                if (__any_sync(0xffffffffu, fresh != 0)) {
+                    // as the two-phase form counts: slots in use when the sub-step began, plus the new ones
+                    int used = held + fresh, any = fresh;
+                    for (int o = 1; o < LPP; o <<= 1) {
+                        used += __shfl_xor_sync(0xffffffffu, used, o);
+                        any += __shfl_xor_sync(0xffffffffu, any, o);
+                    }
+                    if (any && used > room) *fail = 1;
+                }
+                if (walls) {
+                    for (int e = 0; e < NW; ++e) {
+                        const int w = k + e * LPP;
+                        if (!((wnear >> e) & 1)) continue;
+                        const double sep = -(dot3(P.p, d.wall_n + 3 * w) - d.wall_d[w]);
+                        const bool on = (wact >> e) & 1;
+                        if (on && sep > P.rad) {
+                            wact &= ~(1 << e);
+                            wdirty |= 1 << e;
+                        } else if (on || sep <= P.rad) {
+                            double shr[3], cp[3], Fc[3];
+                            for (int t = 0; t < 3; ++t) shr[t] = on ? wsh[e][t] : 0.0;
+                            wall_force(A, P, w, shr, cp, Fc, F, M);
+                            hit = true;
+                            for (int t = 0; t < 3; ++t) {
+                                wsh[e][t] = shr[t];
+                                wcp[e][t] = cp[t];
+                                wF[e][t] = Fc[t];
+                            }
+                            wact |= 1 << e;
+                            wdirty |= 1 << e;
+                        }
+                    }
+                }
+                __syncwarp();
+                const bool hits = __any_sync(0xffffffffu, hit);
+                if (hits) {
+#pragma unroll
+                    for (int o = 1; o < LPP; o <<= 1)
+                        for (int t = 0; t < 3; ++t) {
+                            F[t] += __shfl_xor_sync(0xffffffffu, F[t], o);
+                            M[t] += __shfl_xor_sync(0xffffffffu, M[t], o);
+                        }
+                }
+                // integration, by every lane of the particle alike (integrate_particle, roles 0 and 1); lanes
+                // without a particle stay with their warp (theirs counts as frozen)
+                for (int t = 0; t < 3; ++t) {
+                    double x = F[t] + (s == 0 ? af[t] : 0.0);
+                    x += P.mass * d.g[t];
+                    x += ffl[t];
+                    force[t] = x;
+                    moment[t] = M[t] + (s == 0 ? am[t] : 0.0) + mfl[t];
+                }
+                double x[3] = {P.p[0], P.p[1], P.p[2]}, y[3];
+                if (!frozen) {
+                    translate_update(d.dt, fixed, imass, force, P.p, P.v, acc);
+                    for (int t = 0; t < 3; ++t) y[t] = P.p[t];
+                    wrap_position(d, P.p);
+                    double alpha[3];
+                    if (iso)
+                        for (int t = 0; t < 3; ++t) alpha[t] = moment[t] * iI;
+                    else
+                        angular_general(q, P.w, moment, s_I[g], alpha);
+                    spin_update(d.dt, P.w, wd, alpha);
+                }
+                // publish at once; what no partner waits for comes after
+                if (np_most > 0 && s + 1 < S) {
+                    ulonglong2 *out = flow_packets(f, i, (s + 1) & 1);
+                    const unsigned long long tag = tag0 + s + 1;
+#pragma unroll
+                    for (int t = 0; t < 3; ++t) {
+                        packet_store(nn > 0 && t % LPP == k, out + t, P.p[t], tag);
+                        packet_store(nn > 0 && (3 + t) % LPP == k, out + 3 + t, P.v[t], tag);
+                        packet_store(nn > 0 && (6 + t) % LPP == k, out + 6 + t, P.w[t], tag);
+                    }
+                }
+                if (!frozen) {
+                    quat_update(d.dt, q, P.w);
+                    for (int t = 0; t < 3; ++t) D[t] += y[t] - x[t];
+                    if (y[0] != P.p[0] || y[1] != P.p[1] || y[2] != P.p[2]) {
+                        int c[3];
+                        ref_cell(d, P.p, c);
+                        if (cell_index(d, c[0], c[1], c[2]) < 0) *fail = 1;
+                    }
+                    if (!(dot3(D, D) <= 0.999 * (m * m))) *fail = 1;
+                }
+            }
+            if (late) {
+                atomicOr(d.status, (int)LBDEM_ST_WAIT_TIMEOUT);
+                *fail = 1;
+            }
+            // every block has built by now: clear the lists it read
+            grid_wait(d.sync, gen, d.status);
+            for (int c = me; c < A.ncell; c += nthr) count[c] = 0;
+            if (me == 0) fail_words[(chunk + 1) & 1] = 0;
+            grid_barrier(d.sync, gen, d.status);
+            failed = *fail != 0;
+            if (!failed) {
+                // -------------------------------------------------- commit
+                const size_t base = (size_t)i * d.maxc;
+                int drop = 0, born = 0;
+                if (act) {
+                    if (k == 0) {
+                        for (int t = 0; t < 3; ++t) {
+                            d.pos[3 * i + t] = P.p[t];
+                            d.vel[3 * i + t] = P.v[t];
+                            d.acc[3 * i + t] = acc[t];
+                            d.force[3 * i + t] = force[t];
+                            d.acc_force[3 * i + t] = 0.0;
+                        }
+                        bin_particle(d, i, d.cell_count + (size_t)(parity ^ (S & 1)) * A.ncell);
+                    }
+                    if (k == LPP - 1) {
+                        for (int t = 0; t < 3; ++t) {
+                            d.omega[3 * i + t] = P.w[t];
+                            d.omega_dot[3 * i + t] = wd[t];
+                            d.moment[3 * i + t] = moment[t];
+                            d.acc_moment[3 * i + t] = 0.0;
+                        }
+                        for (int t = 0; t < 4; ++t) d.quat[4 * i + t] = q[t];
+                    }
+                    for (int e = 0; e < NW; ++e) {
+                        if (!((wdirty >> e) & 1)) continue;
+                        const size_t s = (size_t)i * 6 + k + e * LPP;
+                        d.wcf_active[s] = (wact >> e) & 1;
+                        if ((wact >> e) & 1)
+                            for (int t = 0; t < 3; ++t) {
+                                d.wcf_shear[3 * s + t] = wsh[e][t];
+                                d.wcf_pos[3 * s + t] = wcp[e][t];
+                                d.wcf_force[3 * s + t] = wF[e][t];
+                            }
+                    }
+                    // listed contacts in their slots; dropped ones leave gaps
+                    for (int e = 0; e < np; ++e) {
+                        if (pj[e] < i) continue;
+                        const bool on = (pact >> e) & 1u;
+                        if (pslot[e] < 0) {
+                            born += on;
+                        } else if (!on) {
+                            d.cf_active[base + pslot[e]] = 0;
+                            drop = 1;
+                        } else if ((pdirty >> e) & 1u) {
+                            const size_t s = base + pslot[e];
+                            for (int t = 0; t < 3; ++t) {
+                                d.cf_shear[3 * s + t] = psh[e][t];
+                                d.cf_pos[3 * s + t] = pcp[e][t];
+                                d.cf_force[3 * s + t] = pF[e][t];
+                            }
+                        }
+                    }
+                }
+                // close the gaps, then append the new contacts in lane order
+                int before = 0, all = born, drops = drop;
+#pragma unroll
+                for (int o = 1; o < LPP; o <<= 1) {
+                    const int x = __shfl_xor_sync(0xffffffffu, all, o);
+                    before += (k & o) ? x : 0;
+                    all += x;
+                    drops += __shfl_xor_sync(0xffffffffu, drops, o);
+                }
+                __syncwarp();
+                int kept = n_used;
+                if (act && k == 0 && drops) kept = compact_slots(d, i, n_used);
+                __syncwarp();
+                kept = __shfl_sync(0xffffffffu, kept, 0, LPP);
+                if (act) {
+                    int at = kept + before;
+                    for (int e = 0; e < np; ++e) {
+                        if (pj[e] < i || pslot[e] >= 0 || !((pact >> e) & 1u)) continue;
+                        const size_t s = base + at++;
+                        d.cf_j[s] = pj[e];
+                        d.cf_active[s] = 1;
+                        for (int t = 0; t < 3; ++t) {
+                            d.cf_shear[3 * s + t] = psh[e][t];
+                            d.cf_pos[3 * s + t] = pcp[e][t];
+                            d.cf_force[3 * s + t] = pF[e][t];
+                        }
+                    }
+                    if (k == 0 && (drops || all)) d.cfn[i] = kept + all;
+                }
+            } else {
+                // the lists were cleared: bin the untouched positions again
+                if (act && k == 0) bin_particle(d, i, count);
+                grid_barrier(d.sync, gen, d.status);
+            }
+        }
+        if (failed) flow_two_phase<WRAP>(A, parity, S, gen);
+        parity ^= S & 1;
+        done += S;
+        ++chunk;
+        if (done < f.nsub && !failed) grid_barrier(d.sync, gen, d.status);
+    }
+    // leave the barrier and the failure words clear for the next launch
+    if (gridDim.x == 1) {
+        __syncthreads();
+        if (threadIdx.x < 2) fail_words[threadIdx.x] = 0;
+        if (threadIdx.x == 0) *epoch = epoch0 + (unsigned long long)chunk * FLOW_TAGS;
+    } else if (barrier_release(d.sync)) {
+        fail_words[0] = fail_words[1] = 0;
+        *epoch = epoch0 + (unsigned long long)chunk * FLOW_TAGS;
+    }
+}
+
+// The per-material Hertz constants of DemArgs, from
 // hertz.py:45-97 (particle-particle: the restitution 0.5 (e + e)) and
 // hertz.py:99-153 (particle-wall).
 static void contact_constants(DemArgs &A) {
     const lbdem_dem &d = A.d;
     for (int tj = 0; tj < 2; ++tj) {
-        A.hz_ys[tj] = 1.0 / ((1.0 - d.nu[0] * d.nu[0]) / d.E[0] + (1.0 - d.nu[tj] * d.nu[tj]) / d.E[tj]);
-        A.hz_gs[tj] = 1.0 / (2.0 * (2.0 - d.nu[0]) * (1.0 + d.nu[0]) / d.E[0] +
-                             2.0 * (2.0 - d.nu[tj]) * (1.0 + d.nu[tj]) / d.E[tj]);
+        const double Ys = 1.0 / ((1.0 - d.nu[0] * d.nu[0]) / d.E[0] + (1.0 - d.nu[tj] * d.nu[tj]) / d.E[tj]);
+        const double Gs = 1.0 / (2.0 * (2.0 - d.nu[0]) * (1.0 + d.nu[0]) / d.E[0] +
+                                 2.0 * (2.0 - d.nu[tj]) * (1.0 + d.nu[tj]) / d.E[tj]);
         const double e = tj == 0 ? 0.5 * (d.e[0] + d.e[0]) : d.e[1];
         const double lne = log(e);
-        A.hz_beta[tj] = lne / sqrt(lne * lne + M_PI * M_PI);
+        const double beta = lne / sqrt(lne * lne + M_PI * M_PI);
+        A.hz_kn[tj] = 4.0 / 3.0 * Ys;
+        A.hz_kt[tj] = 8.0 * Gs;
+        A.hz_gn[tj] = -2.0 * beta * sqrt(5.0 / 6.0 * 2.0 * Ys);    // Sn = 2 Ys x
+        A.hz_gt[tj] = -2.0 * beta * sqrt(5.0 / 6.0 * 8.0 * Gs);    // St = 8 Gs x
     }
 }
 
@@ -846,14 +1574,14 @@ static thread_local int g_dem_launches = 0;
 // cooperative kernel (128 threads, no dynamic shared memory) on device `dev`:
 // constant for a device, so looked up once per device and form (the host
 // launch of every call would otherwise repeat three driver queries).
-static bool coop_residency(int dev, bool wrap, const void *kcoop, int &coop, int &nsm, int &per_sm) {
+static bool coop_residency(int dev, int form, const void *kcoop, int &coop, int &nsm, int &per_sm) {
     constexpr int MAXDEV = 64;
     static std::mutex mu;
-    static int cached[2][MAXDEV][3];
-    static bool have[2][MAXDEV] = {};
+    static int cached[10][MAXDEV][3];   // form: k_dem_coop without / with images, then the forms of k_dem_flow likewise
+    static bool have[10][MAXDEV] = {};
     if (dev < 0 || dev >= MAXDEV) return false;
     std::lock_guard<std::mutex> lock(mu);
-    if (!have[wrap][dev]) {
+    if (!have[form][dev]) {
         int c = 0, n = 0, p = 0;
         cudaDeviceGetAttribute(&c, cudaDevAttrCooperativeLaunch, dev);
         cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
@@ -861,18 +1589,89 @@ static bool coop_residency(int dev, bool wrap, const void *kcoop, int &coop, int
             cudaGetLastError();
             return false;
         }
-        cached[wrap][dev][0] = c;
-        cached[wrap][dev][1] = n;
-        cached[wrap][dev][2] = p;
-        have[wrap][dev] = true;
+        cached[form][dev][0] = c;
+        cached[form][dev][1] = n;
+        cached[form][dev][2] = p;
+        have[form][dev] = true;
     }
-    coop = cached[wrap][dev][0];
-    nsm = cached[wrap][dev][1];
-    per_sm = cached[wrap][dev][2];
+    coop = cached[form][dev][0];
+    nsm = cached[form][dev][1];
+    per_sm = cached[form][dev][2];
     return true;
 }
 
 int lbdem_dem_launches_last(void) { return g_dem_launches; }
+
+// Forms of the one launch without per-sub-step barriers, in the order of
+// preference: all particles must be resident at once, and the first form that
+// allows it is taken (148 SMs: up to 4736, 9472, 14208 and 28416 particles).
+// 11 sub-steps with the forms that still fit: 8000 spheres of a dense bed, all
+// in contact, 101, 130 and 127 us (two-phase 250); 10,000 of a channel 76 and
+// 87 us (two-phase 210).
+struct FlowForm {
+    int lanes;
+    const void *kern[2];   // without / with periodic images
+};
+constexpr int FLOW_FORMS = 4;
+static const FlowForm flow_forms[FLOW_FORMS] = {
+    {8, {(const void *)k_dem_flow<false, 8, 2>, (const void *)k_dem_flow<true, 8, 2>}},
+    {4, {(const void *)k_dem_flow<false, 4, 2>, (const void *)k_dem_flow<true, 4, 2>}},
+    {4, {(const void *)k_dem_flow<false, 4, 3>, (const void *)k_dem_flow<true, 4, 3>}},
+    {2, {(const void *)k_dem_flow<false, 2, 3>, (const void *)k_dem_flow<true, 2, 3>}},
+};
+
+// The form for D's particles (index), or -1 where none applies.  Periodic axes
+// must be longer than 2.5 broad-phase cells, so that no pair is near both
+// directly and through an image.
+static int flow_form(const lbdem_dem *D, int dev, int *blocks) {
+    if (D->n > 1)
+        for (int a = 0; a < 3; ++a)
+            if (D->periodic[a] && !(D->dom_max[a] - D->dom_min[a] > 2.5 * D->cell_size)) return -1;
+    const bool wrap = D->wrap_pairs != 0;
+    for (int l = 0; l < FLOW_FORMS; ++l) {
+        const int gpb = FLOW_THREADS / flow_forms[l].lanes, nb = (D->n + gpb - 1) / gpb;
+        *blocks = nb;
+        if (nb == 1) return l;
+        int coop = 0, nsm = 0, per_sm = 0;
+        if (!D->sync || !coop_residency(dev, 2 + 2 * l + wrap, flow_forms[l].kern[wrap], coop, nsm, per_sm) || !coop)
+            return -1;
+        if (nb <= per_sm * nsm) return l;
+    }
+    return -1;
+}
+
+int lbdem_dem_substeps_flow(lbdem_dem *D, int32_t nsub, void *work, void *stream) {
+    int rc = check_dem(D);
+    if (rc) return rc;
+    const char *mode = getenv("LBDEM_DEM_KERNELS");
+    int dev = 0, nb = 0, form = -1;
+    cudaGetDevice(&dev);
+    if (work && D->n > 0 && nsub > 0 && (!mode || strcmp(mode, "flow") == 0)) form = flow_form(D, dev, &nb);
+    // (the barrier's arrival counter must stay far from wrapping)
+    if (form < 0 || (nb > 1 && !mode && nsub < FLOW_MIN_SUBSTEPS) || 8ll * nsub * nb >= (1ll << 30))
+        return lbdem_dem_substeps(D, nsub, stream);
+    g_dem_launches = 0;
+    FlowArgs f;
+    f.A.d = *D;
+    f.A.ncell = D->gdim[0] * D->gdim[1] * D->gdim[2];
+    f.A.parity = D->parity;
+    contact_constants(f.A);
+    f.work = static_cast<unsigned char *>(work);
+    f.nsub = nsub;
+    cudaStream_t st = (cudaStream_t)stream;
+    const void *kern = flow_forms[form].kern[D->wrap_pairs != 0];
+    void *args[] = {&f};
+    const int threads = nb > 1 ? FLOW_THREADS : (flow_forms[form].lanes * D->n + 31) / 32 * 32;
+    const cudaError_t e = nb > 1 ? cudaLaunchCooperativeKernel(kern, dim3(nb), dim3(threads), args, 0, st)
+                                 : cudaLaunchKernel(kern, dim3(1), dim3(threads), args, 0, st);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return lbdem_dem_substeps(D, nsub, stream);
+    }
+    D->parity ^= (nsub & 1);
+    g_dem_launches = 1;
+    return check_launch("dem_substeps (flow)");
+}
 
 int lbdem_dem_substeps(lbdem_dem *D, int32_t nsub, void *stream) {
     g_dem_launches = 0;

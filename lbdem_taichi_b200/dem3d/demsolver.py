@@ -217,6 +217,7 @@ class DEMSolver:
         self.acc_force = torch.zeros((max(n, 1), 3), **f64)
         self.acc_moment = torch.zeros((max(n, 1), 3), **f64)
         self.sync = torch.zeros(2, **i32)
+        self.flow = torch.zeros(N.DEM_FLOW_BYTES[0] + N.DEM_FLOW_BYTES[1] * n, dtype=torch.uint8, device=DEV)
         # the reference hashes cells into a 2^k table: distinct cells alias when
         # their coordinates agree in the low bits kept by Morton-code mod 2^k
         T = reference_table_size(rmax, dmin, dmax) if n else 1 << 20
@@ -356,7 +357,7 @@ class DEMSolver:
         if self.n == 0 or nsub <= 0:
             return
         self._ensure_binned()
-        N.call("lbdem_dem_substeps", C.byref(self._d), int(nsub), N.stream_handle())
+        N.call("lbdem_dem_substeps_flow", C.byref(self._d), int(nsub), N.ptr(self.flow), N.stream_handle())
 
     def run_simulation(self):
         """One DEM time step (demsolver.py:848-862)."""
