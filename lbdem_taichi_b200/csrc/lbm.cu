@@ -202,21 +202,18 @@ struct CellForce {
 // images: r - P rint(r / P); with P = 1/P = 0 (no images) it returns r exactly.
 __device__ __forceinline__ float min_image(float r, float P, float iP) { return fmaf(-P, rintf(r * iP), r); }
 
-// PSC quantities of one cell owned by a particle (psclattice3d.py:144-182;
-// B from the current omega as hybridlattice.py:236-245): weight B, 3 u_s,
-// and the cell's force B (j - rho u_s) with its torque about the centre.
-// WRAP: the map has periodic images, lever arms take the minimum image (the
-// branch-free form is the identity where an axis has none).
+// Lever arm of a cell about its owner's centre and the solid velocity there
+// (psclattice3d.py:144-182).  WRAP: the map has periodic images, lever arms
+// take the minimum image (the branch-free form is the identity where an axis
+// has none).
+struct PscGeo {
+    float rx, ry, rz, sx, sy, sz;
+};
 template <bool WRAP>
-__device__ __forceinline__ float psc_cell(const StepArgs &a, uint32_t key, float eps_smooth, float om, float rho,
-                                          float jx, float jy, float jz, int x, int y, int z, float &s3x, float &s3y,
-                                          float &s3z, CellForce &cf) {
-    cf.gid = (int)key_gid(key);
-    const float eps = a.eps ? eps_smooth : ((key & KEY_FULL) ? 1.f : (float)key_count(key) * (1.f / 125.f));
-    const float taum = rcp_fast(om) - 0.5f;
-    const float Bw = eps * taum * rcp_fast((1.f - eps) + taum);
-    const float4 t0 = a.table[4 * cf.gid + 0], t1 = a.table[4 * cf.gid + 1];
-    const float4 t2 = a.table[4 * cf.gid + 2], t3 = a.table[4 * cf.gid + 3];
+__device__ __forceinline__ PscGeo psc_geo(const StepArgs &a, uint32_t key, int x, int y, int z) {
+    const int gid = (int)key_gid(key);
+    const float4 t0 = a.table[4 * gid + 0], t1 = a.table[4 * gid + 1];
+    const float4 t2 = a.table[4 * gid + 2], t3 = a.table[4 * gid + 3];
     // integer part first (exact), then the fractional centre: image cells round as interior ones
     float ix = (float)x - t0.x, iy = (float)y - t0.y, iz = (float)z - t0.z;
     if constexpr (WRAP) {
@@ -224,17 +221,39 @@ __device__ __forceinline__ float psc_cell(const StepArgs &a, uint32_t key, float
         iy = min_image(iy, a.per_y, a.iper_y);
         iz = min_image(iz, a.per_z, a.iper_z);
     }
-    const float rx = ix - t1.x, ry = iy - t1.y, rz = iz - t1.z;
-    const float sx = t2.x + (t3.y * rz - t3.z * ry);
-    const float sy = t2.y + (t3.z * rx - t3.x * rz);
-    const float sz = t2.z + (t3.x * ry - t3.y * rx);
-    s3x = 3.f * sx; s3y = 3.f * sy; s3z = 3.f * sz;
-    cf.hx = Bw * fmaf(-rho, sx, jx);
-    cf.hy = Bw * fmaf(-rho, sy, jy);
-    cf.hz = Bw * fmaf(-rho, sz, jz);
-    cf.tx = ry * cf.hz - rz * cf.hy;
-    cf.ty = rz * cf.hx - rx * cf.hz;
-    cf.tz = rx * cf.hy - ry * cf.hx;
+    PscGeo g;
+    g.rx = ix - t1.x; g.ry = iy - t1.y; g.rz = iz - t1.z;
+    g.sx = t2.x + (t3.y * g.rz - t3.z * g.ry);
+    g.sy = t2.y + (t3.z * g.rx - t3.x * g.rz);
+    g.sz = t2.z + (t3.x * g.ry - t3.y * g.rx);
+    return g;
+}
+
+// Bring an owner's table row to L1 ahead of psc_geo: its loads in the middle
+// of the collision are then hits instead of a second round trip after the
+// gathers' (frozen bed of 128^3 cells, a third of the warps owned: 61.3 to 58.5
+// us).  Loading it early into registers spills eight of the step's 64.
+__device__ __forceinline__ void prefetch_table(const StepArgs &a, uint32_t key) {
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(a.table + 4 * key_gid(key)));
+}
+
+// PSC quantities of one cell owned by a particle: weight B (from the current
+// omega as hybridlattice.py:236-245), 3 u_s, and the cell's force B (j - rho
+// u_s) with its torque about the centre.
+__device__ __forceinline__ float psc_cell(const StepArgs &a, uint32_t key, float eps_smooth, float om, float rho,
+                                          float jx, float jy, float jz, const PscGeo &g, float &s3x, float &s3y,
+                                          float &s3z, CellForce &cf) {
+    cf.gid = (int)key_gid(key);
+    const float eps = a.eps ? eps_smooth : ((key & KEY_FULL) ? 1.f : (float)key_count(key) * (1.f / 125.f));
+    const float taum = rcp_fast(om) - 0.5f;
+    const float Bw = eps * taum * rcp_fast((1.f - eps) + taum);
+    s3x = 3.f * g.sx; s3y = 3.f * g.sy; s3z = 3.f * g.sz;
+    cf.hx = Bw * fmaf(-rho, g.sx, jx);
+    cf.hy = Bw * fmaf(-rho, g.sy, jy);
+    cf.hz = Bw * fmaf(-rho, g.sz, jz);
+    cf.tx = g.ry * cf.hz - g.rz * cf.hy;
+    cf.ty = g.rz * cf.hx - g.rx * cf.hz;
+    cf.tz = g.rx * cf.hy - g.ry * cf.hx;
     return Bw;
 }
 
@@ -255,14 +274,14 @@ __device__ __forceinline__ float psc_cell(const StepArgs &a, uint32_t key, float
 // OVR: collide with the density and velocity in ovr[4] = (rho, ux, uy, uz)
 // instead of the moments of h -- the boundary pass, where a wet-node rule set
 // them (the reference always collides with its rho / vel fields).
+// geo(i): lever arm and solid velocity of cell i (asked for owned cells only).
 // PACK_PSC: the PSC pair updates also run two pairs per f32x2 instruction
 // (same rounding per lane; needs the registers of the row-staged kernel).
-template <class V, int SMAG, bool OVR = false, bool WRAP = false, bool PACK_PSC = false, class HA, class Out,
-          class AuxOut, class Macro>
-__device__ __forceinline__ void collide(const StepArgs &a, const HA &h, const bool act[], const int xs[], int y,
-                                        int z, const V aux[5], bool psc, const uint32_t key[], const float eps[],
-                                        CellForce cf[], Out &&out, AuxOut &&aux_out, Macro &&macro,
-                                        const float *ovr = nullptr) {
+template <class V, int SMAG, bool OVR = false, bool PACK_PSC = false, class HA, class Geo, class Out, class AuxOut,
+          class Macro>
+__device__ __forceinline__ void collide(const StepArgs &a, const HA &h, const bool act[], Geo &&geo, const V aux[5],
+                                        bool psc, const uint32_t key[], const float eps[], CellForce cf[], Out &&out,
+                                        AuxOut &&aux_out, Macro &&macro, const float *ovr = nullptr) {
     using L = Lanes<V>;
     // Opposite pairs (q, q+1), q odd: sp = h_q + h_{q+1}, am = h_q - h_{q+1}.
     // Pair p = (q-1)/2 has direction c_q: p0 (1,0,0), p1 (0,1,0), p2 (0,0,1),
@@ -427,8 +446,8 @@ __device__ __forceinline__ void collide(const StepArgs &a, const HA &h, const bo
     for (int i = 0; i < L::N; ++i) {
         if (key[i]) {
             float sx, sy, sz;
-            L::set(Bw, i, psc_cell<WRAP>(a, key[i], eps[i], L::get(om, i), L::get(rho, i), L::get(jx, i), L::get(jy, i),
-                                   L::get(jz, i), xs[i], y, z, sx, sy, sz, cf[i]));
+            L::set(Bw, i, psc_cell(a, key[i], eps[i], L::get(om, i), L::get(rho, i), L::get(jx, i), L::get(jy, i),
+                                   L::get(jz, i), geo(i), sx, sy, sz, cf[i]));
             L::set(s3x, i, sx); L::set(s3y, i, sy); L::set(s3z, i, sz);
         }
     }
@@ -523,12 +542,8 @@ __device__ __forceinline__ void reduce_forces(const StepArgs &a, CellForce c) {
 // ---------------------------------------------------------------------------
 // fused step, one cell per thread
 // ---------------------------------------------------------------------------
-#ifndef ONE_THREADS
-#define ONE_THREADS 256
-#endif
-#ifndef ONE_MIN_BLOCKS
-#define ONE_MIN_BLOCKS 4
-#endif
+constexpr int ONE_THREADS = 256;
+constexpr int ONE_MIN_BLOCKS = 4;
 
 // Moving walls (VEL_LADD neighbours, lbm_solver3d.py:222-225): the bounced
 // population gains 2 w_q rho (c_q . u_wall)/cs^2, rho being the cell's density
@@ -616,12 +631,11 @@ __device__ __forceinline__ void step_cell(const StepArgs &a, int x, int y, int z
     const bool psc = a.key != nullptr && (psc_given >= 0 ? psc_given != 0 : owners != 0u);
     CellForce cf[1];
     const bool acts[1] = {act};
-    const int xs[1] = {x};
     const uint32_t keys[1] = {key};
     const float epss[1] = {(a.eps != nullptr && key) ? a.eps[cell] : 0.f};
     // post-collision values overwrite h[] and aux[] and are stored together
-    collide<float, SMAG, false, WRAP, PACK_PSC>(
-        a, h, acts, xs, y, z, aux, psc, keys, epss, cf, [&](int q, float v) { h[q] = v; },
+    collide<float, SMAG, false, PACK_PSC>(
+        a, h, acts, [&](int) { return psc_geo<WRAP>(a, key, x, y, z); }, aux, psc, keys, epss, cf, [&](int q, float v) { h[q] = v; },
         [&](int k, float v) { aux[k] = v; },
         [&](float r, float u3x, float u3y, float u3z) {
             // post-stream moments of an exit's / inlet's interior neighbour, read by the boundary pass
@@ -662,10 +676,13 @@ __device__ __forceinline__ void step_at(const StepArgs &a, int x, int y, int z) 
     const uint32_t rs = a.rs;                         // elements per row of populations
     const uint32_t r0 = row * rs;
     const uint32_t own = r0 + xslot((uint32_t)xc_, QB);
-    // Issue the 19 gather loads first (their addresses never depend on the
-    // link mask), then resolve the link mask and re-fetch bounce-back
-    // directions on the few cells next to an obstacle.  One pointer per
-    // upwind (row, x) slot; the direction index is an immediate offset.
+    // The owner key first: it comes from L2 while the gathers come from DRAM, so
+    // an owned cell's table row is asked for (prefetch_table) before the gathers
+    // are waited for.  Then the 19 gather loads (their addresses never depend on
+    // the link mask), then the link mask and a re-fetch of bounce-back
+    // directions on the few cells next to an obstacle.  One pointer per upwind
+    // (row, x) slot; the direction index is an immediate offset.
+    const uint32_t key = (a.key != nullptr) ? a.key[cell] : 0u;
     const T *__restrict__ src = static_cast<const T *>(a.src);
     T raw[Q];
     if (GATHER) {
@@ -696,11 +713,11 @@ __device__ __forceinline__ void step_at(const StepArgs &a, int x, int y, int z) 
 #pragma unroll
         for (int k = 0; k < 5; ++k) aux[k] = lag_ld<T, LAGM>(a, aown, k * 32);
     }
-    uint32_t key = (a.key != nullptr) ? a.key[cell] : 0u;
     // the link mask is read for every cell (a flag that skipped this load for
     // plain blocks cost more -- a dependent load before it -- than the 4 B it
     // saved), unless one value holds for the whole lattice (kernel argument)
     const uint32_t lk = a.links_all ? a.links_all : a.links[cell];
+    if (!STRESS && key) prefetch_table(a, key);   // (the stress form has no register for it: 64.8 against 63.8 us)
     step_cell<T, GATHER, SMAG, WRAP, STRESS, false, LAGM>(a, x, y, z, inb, cell, own, aown, raw, aux, key, lk);
 }
 
@@ -1108,13 +1125,12 @@ __global__ void __launch_bounds__(ROW_THREADS / 2 + 32, ROW2_MIN_BLOCKS) k_psc_s
             const bool psc = psc_warp && (owners & ((threadIdx.x & 16u) ? 0xFFFF0000u : 0x0000FFFFu)) != 0u;
             CellForce cf[2];
             const bool acts[2] = {act, act};
-            const int xs[2] = {x0, x0 + 1};
             const uint32_t keys[2] = {k0, k1};
             const float epss[2] = {0.f, 0.f};
             uint32_t *d = reinterpret_cast<uint32_t *>(static_cast<T *>(a.dst) + own);
             const PairRow<T> hrow{raw};
-            collide<float2, SMAG, false, WRAP>(
-                a, hrow, acts, xs, y, z, aux, psc, keys, epss, cf,
+            collide<float2, SMAG>(
+                a, hrow, acts, [&](int i) { return psc_geo<WRAP>(a, keys[i], x0 + i, y, z); }, aux, psc, keys, epss, cf,
                 [&](int q, float2 v) {
                     if (act) d[q * 16] = Pair16<T>::narrow(v);
                 },
@@ -1527,13 +1543,13 @@ __global__ void __launch_bounds__(128) k_boundary(const StepArgs a, const uint32
     const bool psc = a.key != nullptr && __any_sync(0xffffffffu, key != 0u);
     CellForce cf[1];
     const bool acts[1] = {act};
-    const int xs[1] = {x};
     const uint32_t keys[1] = {key};
     const float epss[1] = {(a.eps != nullptr && key) ? a.eps[cell] : 0.f};
     const float ovr[4] = {rho, u[0], u[1], u[2]};
     float hout[Q];
-    collide<float, SMAG, true, true>(
-        a, h, acts, xs, y, z, aux, psc, keys, epss, cf, [&](int q, float v) { hout[q] = v; },
+    collide<float, SMAG, true>(
+        a, h, acts, [&](int) { return psc_geo<true>(a, key, x, y, z); }, aux, psc, keys, epss, cf,
+        [&](int q, float v) { hout[q] = v; },
         [&](int k, float v) { aux[k] = v; }, [](float, float, float, float) {}, ovr);
     // an inlet's post-collision populations are read only by free-slip mirrors
     if (act && (rule != WET_INLET || a.slip)) {
@@ -1957,13 +1973,25 @@ static void set_periods(StepArgs &a, const lbdem_psc *P) {
     a.wrap_any = a.per_x > 0.f || a.per_y > 0.f || a.per_z > 0.f;
 }
 
-static void step_geometry(const lbdem_lattice *L, dim3 &grid, dim3 &block, int nthreads = 256) {
-    int bx = ((L->nx + 31) / 32) * 32;
-    if (bx > nthreads) bx = nthreads;
-    int by = nthreads / bx;
-    if (by > L->ny) by = L->ny;
-    block = dim3(bx, by, 1);
-    grid = dim3((L->nx + bx - 1) / bx, (L->ny + by - 1) / by, L->nz);
+// Blocks of w x-blocks (32 w threads) by `by` rows, w by = 8 warps: the split
+// of 8 that leaves the fewest warps past the row's end and the last row, wider
+// ones first.  Idle warps hold their registers until their block ends: 362 x
+// 122 x 122 cells (12 x-blocks a row) in blocks of 8 x-blocks left 4 of 16
+// warps idle and took 0.291 ms, in blocks of 4 x 2 0.212 ms.
+static void step_geometry(const lbdem_lattice *L, dim3 &grid, dim3 &block) {
+    const unsigned nb = (unsigned)(L->nx + 31) / 32, ny = (unsigned)L->ny;
+    unsigned w = 0, best = 0;
+    for (unsigned c = 8; c >= 1; c >>= 1) {
+        const unsigned rows = 8 / c, cols = (nb + c - 1) / c;
+        const unsigned warps = cols * c * ((ny + rows - 1) / rows * rows);
+        if (w == 0 || warps < best) {
+            w = c;
+            best = warps;
+        }
+    }
+    const unsigned rows = std::min(8 / w, ny);
+    block = dim3(32 * w, rows, 1);
+    grid = dim3((nb + w - 1) / w, (ny + rows - 1) / rows, (unsigned)L->nz);
 }
 
 // ---------------------------------------------------------------------------
@@ -2167,7 +2195,7 @@ static int launch_step(const lbdem_lattice *L, const lbdem_psc *P, const lbdem_g
         a.stress_out = L->stress;
     }
     dim3 grid, block;
-    step_geometry(L, grid, block, ONE_THREADS);
+    step_geometry(L, grid, block);
     // FP16 lagged state exists under FP32 storage only (fill_args checks)
     constexpr int LAG_H = sizeof(T) == 4 ? LAG_HALF : LAG_STORE;
 #define LBDEM_STEP_CASE(G_, S_)                                                          \
