@@ -22,7 +22,7 @@ struct MapArgs {
     int table_in_scatter;    // no clearing pass runs: the scatter writes the table and resets the forces
     double dx, dt, xmin, ymin, zmin;
     const double *pos, *radius, *vel, *omega;
-    const uint32_t *links;
+    const uint32_t *links;   // NULL: no cell is left out (one link mask for the lattice, all FLUID)
     uint32_t *key;
     float4 *table;
     double *prev;
@@ -168,12 +168,56 @@ __device__ __forceinline__ bool subcell_inside_exact(double xc, double yc, doubl
 //     both sides of the surface go to a shared list (those with none inside
 //     are dropped).
 //  2. one thread per partial cell counts its 5^3 sub-points
-//     (psclattice3d.py:121-131) from the squared per-axis offsets; the few
-//     cells with a sub-point near the surface are recounted one warp per
-//     cell (25 lanes x 5, __reduce_add_sync).  A sub-point whose
-//     FP32 squared distance lies within 1e-4 (1 + r^2) of r^2 is re-tested
-//     with the reference's exact FP64 expression (|s32 - s64| < 2e-5 (1 + r^2)
-//     for these offsets), so counts are bit-exact.
+//     (psclattice3d.py:121-131) in FP32, column by column (count_columns; below
+//     COUNT_COLUMNS_R from the squared per-axis offsets); the few cells with a
+//     sub-point near the surface are recounted one warp per cell (25 lanes x 5,
+//     __reduce_add_sync), where a sub-point whose FP32 squared distance lies
+//     within 1e-4 (1 + r^2) of r^2 is re-tested with the reference's exact FP64
+//     expression, so counts are bit-exact.
+// The count of a partial cell is the kernel: 500 instructions as 2 x 125
+// comparisons, for some 450 cells a sphere of diameter 10.  Here a column of
+// five sub-points along the axis of the largest centre offset a (all three
+// offsets taken positive: the sub-points are symmetric) is one square root: with
+// w the half chord of the column, the points a + 0.2 k - 0.4 below w are the
+// k < u = 5 (w - a) + 2, i.e. ceil(u) of them, clamped to 0 .. 5 -- ten
+// instructions.  a >= (r - 0.87) / sqrt(3) is above 0.65 for r >= 2, so the far side of
+// the sphere never cuts the column.  *edge receives the largest distance of
+// u + 1/2 from an integer: 1/2 where a point lies on the surface.  FP32 errors:
+// offsets (r + 2) 2^-24, squares and sums 3 2^-24 (r + 1)^2, root 2^-21
+// relative, together below 3e-6 (1 + r^2) in the squared distance; a cell is
+// recounted when a point is within 2e-5 (1 + r^2) (5 / 2 of that over w in u,
+// w >= a - 0.4 at a crossing).
+constexpr double COUNT_COLUMNS_R = 2.0;
+__device__ __forceinline__ int count_columns(const float4 &o, float rr25, float *edge) {
+    float a = fabsf(o.x), b = fabsf(o.y), c = fabsf(o.z), t;
+    t = fmaxf(a, b); b = fminf(a, b); a = t;
+    t = fmaxf(a, c); c = fminf(a, c); a = t;
+    b *= 5.f; c *= 5.f;
+    constexpr float SPAN = 5.4f;                           // u + 1/2 in 0 .. 5.4 as 0 .. 1: the clamp is the .sat
+    const float off = (2.5f - 5.f * a) * (1.f / SPAN);
+    float c2[5];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) c2[m] = (c + (float)(m - 2)) * (c + (float)(m - 2));
+    int bits = 0;
+    float e = 0.f;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+        const float rb = rr25 - (b + (float)(i - 2)) * (b + (float)(i - 2));
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            const float q = fmaxf(rb - c2[j], 1e-12f);     // (5 w)^2
+            float rs;
+            asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(q));
+            const float v = __saturatef(fmaf(q * rs, 1.f / SPAN, off));
+            const float m = fmaf(v, SPAN, 12582912.f);     // 1.5 2^23: the low bits are rint(u + 1/2)
+            bits += __float_as_int(m) - 0x4B400000;
+            e = fmaxf(e, fabsf(fmaf(v, SPAN, 12582912.f - m)));
+        }
+    }
+    *edge = e;
+    return bits;
+}
+
 constexpr int MAP_CHUNK = 2048;         // box cells classified per round (shared-memory lists)
 constexpr int MAP_THREADS = 256;
 constexpr int MAP_MIN_BLOCKS = 5;       // per SM (46 registers, 40 KB of shared memory each)
@@ -224,6 +268,10 @@ __global__ void __launch_bounds__(MAP_THREADS, WRAP ? 4 : MAP_MIN_BLOCKS) k_map_
         const float all2 = t_all > 0.0 ? (float)(t_all * t_all) : -1.f, marg_a = (float)(1e-4 * (1.0 + t_all * t_all));
         const float none2 = (float)(t_none * t_none), marg_n = (float)(1e-4 * (1.0 + t_none * t_none));
         const float lo = (float)rr - band, hi = (float)rr + band;
+        const bool columns = r >= COUNT_COLUMNS_R;
+        const float rr25 = (float)(25.0 * rr);
+        const float edge_max = 0.5f - (float)(2.5 * 2e-5 * (1.0 + rr) / ((r - 0.8661) / 1.7320509 - 0.4));
+        const float bx = (float)(xc - (double)x0), by = (float)(yc - (double)y0), bz = (float)(zc - (double)z0);
         const unsigned tot = (unsigned)ex * (unsigned)ey * (unsigned)ez;
         // this block's range of the box's cells
         const unsigned per = (tot + gridDim.y - 1) / gridDim.y;
@@ -242,14 +290,15 @@ __global__ void __launch_bounds__(MAP_THREADS, WRAP ? 4 : MAP_MIN_BLOCKS) k_map_
             const unsigned lim = min(end, base + MAP_CHUNK);
             for (unsigned t = base + threadIdx.x; t < lim; t += bd) {
                 const int i = x0 + ix, j = y0 + jy, k = z0 + kz;
+                const float fx = bx - (float)ix, fy = by - (float)jy, fz = bz - (float)kz;
                 ix += adx; jy += ady; kz += adz;
                 if (ix >= ex) { ix -= ex; ++jy; }
                 if (jy >= ey) { jy -= ey; ++kz; }
-                const float fx = (float)(xc - (double)i), fy = (float)(yc - (double)j), fz = (float)(zc - (double)k);
+                // (the integer part is exact: bx is a multiple of its own ulp, larger than the result's)
                 const float d2 = (fx * fx + fy * fy) + fz * fz;
                 if (d2 > out2 + marg_o) continue;                 // certainly dist >= t_out
                 const unsigned c = ((unsigned)k * (unsigned)a.ny + (unsigned)j) * (unsigned)a.nx + (unsigned)i;
-                if (a.links[c] & LINK_MAP_SKIP) continue;
+                if (a.links != nullptr && (a.links[c] & LINK_MAP_SKIP)) continue;
                 int full;
                 if (d2 < in2 - marg_i) {
                     full = 1;                                     // certainly dist <= t_in
@@ -272,13 +321,25 @@ __global__ void __launch_bounds__(MAP_THREADS, WRAP ? 4 : MAP_MIN_BLOCKS) k_map_
             }
             __syncthreads();
             const int n = s_n;
-            // 2a. one thread per partial cell: 25 columns x 5 sub-points from the
-            // squared per-axis offsets (-fmad=false).  Per column (x, y) the five
-            // z terms are compared with lo - s_xy and hi - s_xy (their rounding is
-            // far inside the band), so a point counts when its squared distance is
-            // certainly below r^2 and the cell is ambiguous when a point lies
-            // between the two thresholds (the two counts differ); ambiguous cells
-            // go to a second list for an exact warp recount.
+            // 2a. one thread per partial cell; ambiguous cells go to a second list for
+            // an exact warp recount
+            if (columns) {
+                for (int e = threadIdx.x; e < n; e += bd) {
+                    const float4 o = s_off[e];
+                    float edge;
+                    const int cnt = count_columns(o, rr25, &edge);
+                    if (edge > edge_max) s_amb[atomicAdd(&s_na, 1)] = e;
+                    else if (cnt > 0)   // eps = 0 never beats the empty cell (strict >)
+                        atomicMax(a.key + __float_as_uint(o.w), ((uint32_t)cnt << 24) | gbits);
+                }
+            }
+            // small spheres: 25 columns x 5 sub-points from the squared per-axis offsets
+            // (-fmad=false).  Per column (x, y) the five z terms are compared with
+            // lo - s_xy and hi - s_xy (their rounding is far inside the band), so a
+            // point counts when its squared distance is certainly below r^2 and the
+            // cell is ambiguous when a point lies between the two thresholds (the two
+            // counts differ).
+            else
             for (int e = threadIdx.x; e < n; e += bd) {
                 const float4 o = s_off[e];
                 float ox2[5], oy2[5], oz2[5];
@@ -522,7 +583,7 @@ extern "C" int lbdem_psc_map(const lbdem_lattice *L, lbdem_psc *P, const lbdem_g
     a.n = G->n; a.nx = L->nx; a.ny = L->ny; a.nz = L->nz;
     a.dx = P->dx; a.dt = P->dt; a.xmin = P->xmin; a.ymin = P->ymin; a.zmin = P->zmin;
     a.pos = G->pos; a.radius = G->radius; a.vel = G->vel; a.omega = G->omega;
-    a.links = L->links;
+    a.links = L->links_all && !(L->links_all & LINK_MAP_SKIP) ? nullptr : L->links;
     a.key = P->key;
     a.table = (float4 *)P->table;
     a.prev = P->prev;

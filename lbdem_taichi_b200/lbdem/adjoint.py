@@ -82,7 +82,9 @@ class FrozenBedDrag:
         lat.initialize()
         self._ckpt = {0: lat._f[lat._cur].clone()}
         for n in range(1, self.n_steps + 1):
-            lat.collide()
+            # the bed is frozen: initialize() mapped it for every step; the last one maps again, which resets
+            # the force accumulators that the loss is read from
+            lat.collide() if n == self.n_steps else lat._collide_mapped()
             lat.stream()
             if n % self.K == 0 and n < self.n_steps:
                 self._ckpt[n] = lat._f[lat._cur].clone()
@@ -109,14 +111,14 @@ class FrozenBedDrag:
         bbar = torch.zeros(lat.ncells, dtype=torch.float32, device="cuda")
         gbar = torch.zeros(3, dtype=torch.float64, device="cuda")
         dirv = (C.c_double * 3)(*self.direction)
-        states = [torch.empty_like(like) for _ in range(self.K)]
+        states = [None] + [torch.empty_like(like) for _ in range(self.K - 1)]
         cur = 0
         N_ = self.n_steps
         seg_starts = list(range(0, N_, self.K))
         for s0 in reversed(seg_starts):
             s1 = min(s0 + self.K, N_)
-            # states[i] = populations read by step s0 + 1 + i
-            states[0].copy_(self._ckpt[s0])
+            # states[i] = populations read by step s0 + 1 + i (the first are the checkpoint itself)
+            states[0] = self._ckpt[s0]
             for i in range(1, s1 - s0):
                 self._step(Ld, states[i - 1], states[i], gather=(s0 + i) >= 2)
             for n in range(s1, s0, -1):

@@ -170,6 +170,12 @@ class PSCLattice3D(LatticeEngine):
         """Map grains, PSC/BGK collision and force reduction (psclattice3d.py:187-218),
         fused with the pending stream."""
         self.grains2lattice()
+        self._collide_mapped()
+
+    def _collide_mapped(self):
+        """collide() on the map as it is: for particles that have not changed since
+        grains2lattice() or initialize().  Their forces are added to the accumulators,
+        which only a map resets."""
         if self._hydro is not None:
             self._hydro.zero_()
         if self.dem.n > 0:
