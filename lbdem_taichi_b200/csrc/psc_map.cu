@@ -12,9 +12,17 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace lbdem {
+
+// Fewer particles than this: several blocks share a particle's box (148 SMs x 8).
+constexpr int MAP_SPLIT_BELOW = 1184;
+static unsigned map_split(int n) {
+    return (unsigned)(n >= MAP_SPLIT_BELOW ? 1 : std::min(16, (MAP_SPLIT_BELOW + n - 1) / n));
+}
 
 struct MapArgs {
     int n, nx, ny, nz;
@@ -45,10 +53,42 @@ constexpr double SUB_REACH = 0.6928204;
 __device__ __forceinline__ void particle_lattice(const MapArgs &a, int g, double &xc, double &yc, double &zc,
                                                  double &r) {
     // psclattice3d.py:102-105
-    xc = (a.pos[3 * g + 0] - a.xmin + 0.5 * a.dx) / a.dx;
-    yc = (a.pos[3 * g + 1] - a.ymin + 0.5 * a.dx) / a.dx;
-    zc = (a.pos[3 * g + 2] - a.zmin + 0.5 * a.dx) / a.dx;
-    r = (a.radius[g] - 0.5 * a.dx) / a.dx;
+    xc = a.pos[3 * g + 0] - a.xmin + 0.5 * a.dx;
+    yc = a.pos[3 * g + 1] - a.ymin + 0.5 * a.dx;
+    zc = a.pos[3 * g + 2] - a.zmin + 0.5 * a.dx;
+    r = a.radius[g] - 0.5 * a.dx;
+    if (a.dx != 1.0) {   // (a division by one changes no bit, and the four cost 200 instructions)
+        xc /= a.dx;
+        yc /= a.dx;
+        zc /= a.dx;
+        r /= a.dx;
+    }
+}
+
+// (x, y, z) of cell t of a box of tot cells, ex by ey per layer.  FP32 quotients
+// with a correction for boxes of up to 2^21 cells (an integer division is some
+// twenty instructions, and each thread needs eight).
+__device__ __forceinline__ void box_index(unsigned t, unsigned ex, unsigned ey, unsigned tot, int &x, int &y, int &z) {
+    const unsigned exy = ex * ey;
+    unsigned k, j;
+    if (tot < (1u << 21) && t < (1u << 22)) {
+        k = (unsigned)__fdividef((float)t + 0.5f, (float)exy);
+        int rem = (int)(t - k * exy);
+        if (rem < 0) { rem += (int)exy; --k; }
+        else if (rem >= (int)exy) { rem -= (int)exy; ++k; }
+        j = (unsigned)__fdividef((float)rem + 0.5f, (float)ex);
+        int r2 = rem - (int)(j * ex);
+        if (r2 < 0) { r2 += (int)ex; --j; }
+        else if (r2 >= (int)ex) { r2 -= (int)ex; ++j; }
+        x = r2;
+    } else {
+        k = t / exy;
+        const unsigned rem = t - k * exy;
+        j = rem / ex;
+        x = (int)(rem - j * ex);
+    }
+    y = (int)j;
+    z = (int)k;
 }
 
 // Image shifts of a sphere centre c with reach `reach` along `axis`: 0, plus
@@ -93,7 +133,7 @@ template <bool WRAP>
 __global__ void __launch_bounds__(128) k_map_clear(const MapArgs a) {
     const int g = blockIdx.x;
     bool clear = a.have_prev != 0;
-    if (a.disp_limit > 0.0 && a.have_prev && threadIdx.x == 0) {
+    if (a.disp_limit > 0.0 && a.have_prev && threadIdx.x == 0 && blockIdx.y == 0) {
         // pipelined stepping: the near-block mask assumed at most disp_limit
         double xc, yc, zc, r;
         particle_lattice(a, g, xc, yc, zc, r);
@@ -104,7 +144,7 @@ __global__ void __launch_bounds__(128) k_map_clear(const MapArgs a) {
             atomicOr(a.status, (int)LBDEM_ST_PIPELINE_MARGIN);
     }
     if (a.moved != nullptr) {
-        if (g == 0 && threadIdx.x == 0) *a.moved_next = 0u;
+        if (g == 0 && threadIdx.x == 0 && blockIdx.y == 0) *a.moved_next = 0u;
         double xc, yc, zc, r;
         particle_lattice(a, g, xc, yc, zc, r);
         const double *p = a.prev + 4 * (size_t)g;
@@ -134,7 +174,8 @@ __global__ void __launch_bounds__(128) k_map_clear(const MapArgs a) {
             if (ex > 0 && ey > 0 && ez > 0) {
                 const unsigned exy = (unsigned)ex * (unsigned)ey, tot = exy * (unsigned)ez;
                 const float lim2 = (float)(lim * lim) + 1e-3f;
-                for (unsigned t = threadIdx.x; t < tot; t += blockDim.x) {
+                const unsigned per = (tot + gridDim.y - 1) / gridDim.y, beg = blockIdx.y * per;
+                for (unsigned t = beg + threadIdx.x; t < min(tot, beg + per); t += blockDim.x) {
                     const unsigned kz = t / exy, rem = t - kz * exy, jy = rem / (unsigned)ex;
                     const int i = x0 + (int)(rem - jy * (unsigned)ex), j = y0 + (int)jy, k = z0 + (int)kz;
                     const float ddx = (float)(pxc - i), ddy = (float)(pyc - j), ddz = (float)(pzc - k);
@@ -144,7 +185,7 @@ __global__ void __launch_bounds__(128) k_map_clear(const MapArgs a) {
             }
         }
     }
-    if (threadIdx.x == 0 && !a.keys_only) particle_table(a, g);
+    if (threadIdx.x == 0 && blockIdx.y == 0 && !a.keys_only) particle_table(a, g);
 }
 
 // Exact FP64 sub-cell test, in the reference's operation order
@@ -157,7 +198,7 @@ __device__ __forceinline__ bool subcell_inside_exact(double xc, double yc, doubl
     return sqrt((ox * ox + oy * oy) + oz * oz) < r;
 }
 
-// One block per particle -- or, with few particles, gridDim.y blocks sharing
+// One block per particle -- or, with few particles (map_split), gridDim.y blocks sharing
 // its bounding box in contiguous ranges of cells, so that a lone sphere does
 // not map on one SM -- two phases per chunk of the box:
 //  1. each thread classifies one cell -- outside / fully covered / partial
@@ -218,15 +259,16 @@ __device__ __forceinline__ int count_columns(const float4 &o, float rr25, float 
     return bits;
 }
 
-constexpr int MAP_CHUNK = 2048;         // box cells classified per round (shared-memory lists)
-constexpr int MAP_THREADS = 256;
-constexpr int MAP_MIN_BLOCKS = 5;       // per SM (46 registers, 40 KB of shared memory each)
-constexpr int MAP_SPLIT_BELOW = 592;   // 148 SMs x 4 blocks
+constexpr int MAP_CHUNK = 1024;         // box cells classified per round (shared-memory lists)
+constexpr int MAP_THREADS = 128;
+constexpr int MAP_MIN_BLOCKS = 10;      // per SM (48 registers, 20 KB of shared memory each)
 
-// Five 256-thread blocks per SM (46 registers, 40 KB of shared memory each);
-// the image form keeps four (it would spill at five).
+// Ten 128-thread blocks per SM (48 registers, 20 KB of shared memory each); the
+// image form keeps eight (it would spill).  Each thread repeats the sphere's
+// set-up, so that four warps a block instead of eight took 10,000 spheres of
+// diameter 8 from 145 to 116 us and 2000 of diameter 10 from 44 to 41.
 template <bool WRAP>
-__global__ void __launch_bounds__(MAP_THREADS, WRAP ? 4 : MAP_MIN_BLOCKS) k_map_scatter(const MapArgs a) {
+__global__ void __launch_bounds__(MAP_THREADS, WRAP ? 8 : MAP_MIN_BLOCKS) k_map_scatter(const MapArgs a) {
     __shared__ float4 s_off[MAP_CHUNK];   // (xc - i, yc - j, zc - k) in FP32; w = global cell index
     __shared__ int s_amb[MAP_CHUNK];      // partial cells needing the exact recount (index into s_off)
     __shared__ int s_n, s_na;
@@ -279,11 +321,9 @@ __global__ void __launch_bounds__(MAP_THREADS, WRAP ? 4 : MAP_MIN_BLOCKS) k_map_
         // this thread's first cell, then advance by blockDim cells with carries
         // (every chunk but the last is a whole number of blockDim steps)
         const unsigned bd = blockDim.x;
-        const int adx = (int)(bd % (unsigned)ex), ady = (int)((bd / (unsigned)ex) % (unsigned)ey);
-        const int adz = (int)(bd / ((unsigned)ex * (unsigned)ey));
-        const unsigned t0 = beg + threadIdx.x;
-        int ix = (int)(t0 % (unsigned)ex), jy = (int)((t0 / (unsigned)ex) % (unsigned)ey);
-        int kz = (int)(t0 / ((unsigned)ex * (unsigned)ey));
+        int adx, ady, adz, ix, jy, kz;
+        box_index(bd, (unsigned)ex, (unsigned)ey, tot, adx, ady, adz);
+        box_index(beg + threadIdx.x, (unsigned)ex, (unsigned)ey, tot, ix, jy, kz);
         for (unsigned base = beg; base < end; base += MAP_CHUNK) {
             if (threadIdx.x == 0) s_n = s_na = 0;
             __syncthreads();
@@ -609,17 +649,16 @@ extern "C" int lbdem_psc_map(const lbdem_lattice *L, lbdem_psc *P, const lbdem_g
         a.moved_next = P->map_moved + (1 - par);
         P->map_parity = 1 - par;
     }
-    // fewer particles than about four blocks per SM: split each box over several blocks
-    const dim3 sgrid((unsigned)G->n, (unsigned)(G->n >= MAP_SPLIT_BELOW ? 1 : min(16, (MAP_SPLIT_BELOW + G->n - 1) / G->n)));
+    const dim3 sgrid((unsigned)G->n, map_split(G->n));
     // with nothing to clear or check (keys cleared ahead by lbdem_psc_map_clear,
     // or the first map) the scatter writes the table itself: one launch
     const bool clear_pass = a.have_prev || a.moved != nullptr || a.disp_limit > 0.0;
     a.table_in_scatter = !clear_pass;
     if (a.wrap[0] || a.wrap[1] || a.wrap[2]) {
-        if (clear_pass) k_map_clear<true><<<G->n, 128, 0, st>>>(a);
+        if (clear_pass) k_map_clear<true><<<sgrid, 128, 0, st>>>(a);
         k_map_scatter<true><<<sgrid, MAP_THREADS, 0, st>>>(a);
     } else {
-        if (clear_pass) k_map_clear<false><<<G->n, 128, 0, st>>>(a);
+        if (clear_pass) k_map_clear<false><<<sgrid, 128, 0, st>>>(a);
         k_map_scatter<false><<<sgrid, MAP_THREADS, 0, st>>>(a);
     }
     P->have_prev = 1;
@@ -649,8 +688,9 @@ extern "C" int lbdem_psc_map_clear(const lbdem_lattice *L, lbdem_psc *P, const l
         a.period[t] = P->period[t];
     }
     cudaStream_t st = (cudaStream_t)stream;
-    if (a.wrap[0] || a.wrap[1] || a.wrap[2]) k_map_clear<true><<<G->n, 128, 0, st>>>(a);
-    else k_map_clear<false><<<G->n, 128, 0, st>>>(a);
+    const dim3 grid((unsigned)G->n, map_split(G->n));
+    if (a.wrap[0] || a.wrap[1] || a.wrap[2]) k_map_clear<true><<<grid, 128, 0, st>>>(a);
+    else k_map_clear<false><<<grid, 128, 0, st>>>(a);
     P->have_prev = 0;
     return check_launch("psc_map_clear");
 }
