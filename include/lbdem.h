@@ -426,6 +426,20 @@ int lbdem_dem_substeps(lbdem_dem *D, int32_t nsub, void *stream);
 #define LBDEM_DEM_FLOW_BYTES(n) (256 + 512 * (size_t)(n))
 int lbdem_dem_substeps_flow(lbdem_dem *D, int32_t nsub, void *work, void *stream);
 
+/* nsteps coupled steps in one call: per step lbdem_psc_map, the fused step
+ * (src, then alternating; gather for the first, 1 after) and nsub sub-steps of
+ * lbdem_dem_substeps_flow(D, nsub, dem_work) -- the driver loop's collide();
+ * stream(); run_simulation() x nsub, with the same results.  moving = 1 where
+ * particles move: every step but the last zeroes the owner keys that it has
+ * read, instead of a clearing pass of the next map (0 keeps the keys for map
+ * reuse; lattices with open boundaries are to pass 0).  P->hydro_out is zeroed before each step.  The exact map only
+ * (P->eps NULL), P->disp_limit = 0, L->stress NULL, G->n > 0; D must be binned
+ * (lbdem_dem_bin).  *done receives the steps taken (population buffers
+ * swapped), *launches the kernels launched (host memory). */
+int lbdem_psc_run(const lbdem_lattice *L, lbdem_psc *P, const lbdem_grains *G, lbdem_dem *D, void *dem_work,
+                  int32_t nsteps, int32_t nsub, int32_t src, int32_t gather, int32_t moving, int32_t *done,
+                  int32_t *launches, void *stream);
+
 /* FP64 totals over the updated (non-skipped) cells of population buffer
  * f[buf]: out[0] = sum of rho, out[1..3] = sum of momentum.  Valid in either
  * state of the buffer (post-stream or post-collision: streaming conserves

@@ -108,6 +108,8 @@ EXPORTS = {
     "lbdem_psc_near_blocks": ([vp, vp, vp, C.c_double, vp, vp, vp, vp], C.c_int),
     "lbdem_psc_step_phase": ([vp, vp, vp, C.c_int32, C.c_int32, C.c_int32, vp, vp, C.c_uint32, vp], C.c_int),
     "lbdem_psc_map_clear": ([vp, vp, vp, vp], C.c_int),
+    "lbdem_psc_run": ([vp, vp, vp, vp, vp, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32,
+                       C.POINTER(C.c_int32), C.POINTER(C.c_int32), vp], C.c_int),
 }
 
 _lib = None
@@ -166,6 +168,11 @@ def _map_launches(arg):
     if P is None or P.have_prev or P.disp_limit > 0.0:
         return 2
     return 1
+
+
+def count_launches(n: int):
+    """Kernels of a call that reports its own number (lbdem_psc_run)."""
+    _launches[0] += n
 
 
 def call(name: str, *args):

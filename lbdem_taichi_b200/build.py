@@ -7,6 +7,7 @@ Each translation unit is compiled separately:
   psc_map.cu  particle -> lattice mapping, FP64, -fmad=false (bit-exact counts)
   dem.cu      DEM sub-step, FP64, -fmad=false (reference operation order)
   adjoint.cu  reverse mode of the step on a frozen bed (drag gradients)
+  run.cu      the coupled loop's launches
 and linked into one shared library with a static CUDA runtime.
 """
 from __future__ import annotations
@@ -28,6 +29,7 @@ UNITS = {
     "psc_map.cu": ["-fmad=false"],
     "dem.cu": ["-fmad=false"],
     "adjoint.cu": [],
+    "run.cu": [],
 }
 
 

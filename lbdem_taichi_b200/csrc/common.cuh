@@ -141,8 +141,40 @@ constexpr uint32_t KEY_FULL = 1u << 31;
 __host__ __device__ inline uint32_t key_gid(uint32_t k) { return 0xFFFFFFu - (k & 0xFFFFFFu); }
 __host__ __device__ inline int key_count(uint32_t k) { return (int)((k >> 24) & 0x7Fu); }
 
+// Kernels of a coupled step follow one another on one stream, most of them
+// microseconds long on small lattices, with some 2 us between two of them.
+// launch_chained launches a kernel so that its blocks may start once all blocks
+// of the kernel before it have (programmatic dependent launch); grid_dependency,
+// its first statement, waits for that kernel to end and its writes to be
+// visible, then lets the next kernel's blocks come.  After anything but such a
+// kernel it is an ordinary launch.  Not for the fused step: overlapping the map
+// scatter it would keep that kernel's shared-memory split of L1, and its loads
+// in flight need the L1 (0.66 ms against 0.48 at 256^3).
+__device__ __forceinline__ void grid_dependency() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Host-side error reporting
 void set_error(const char *fmt, ...);
 int check_launch(const char *what);
+
+// the fused step with the choice of clearing the keys that it reads (lbm.cu)
+int psc_step(const lbdem_lattice *L, const lbdem_psc *P, const lbdem_grains *G, int src, int gather, bool clear_keys,
+             cudaStream_t st);
 
 }  // namespace lbdem

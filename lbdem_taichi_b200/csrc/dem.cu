@@ -516,6 +516,7 @@ __device__ __forceinline__ void contact_lane(const DemArgs &A, const int32_t *co
 
 template <bool WRAP>
 __global__ void __launch_bounds__(128) k_contacts(const __grid_constant__ DemArgs A) {
+    grid_dependency();
     contact_lane<WRAP>(A, A.d.cell_count + (size_t)A.parity * A.ncell, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -601,6 +602,7 @@ __device__ void integrate_particle(const lbdem_dem &d, int ncell, int parity, in
 __device__ __forceinline__ void integrate_unit(const lbdem_dem &d, int ncell, int parity, int u);
 
 __global__ void __launch_bounds__(128) k_integrate(const __grid_constant__ DemArgs A) {
+    grid_dependency();
     const lbdem_dem &d = A.d;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     // clear the counts consumed by this sub-step (the other half receives the new binning)
@@ -770,6 +772,7 @@ __global__ void __launch_bounds__(512) k_dem_cluster(const __grid_constant__ Dem
 // without the cluster form's register cap (512 threads), so nothing spills.
 template <bool WRAP>
 __global__ void __launch_bounds__(128) k_dem_block(const __grid_constant__ DemArgs A, int nsub) {
+    grid_dependency();
     const lbdem_dem &d = A.d;
     const int nthr = (int)blockDim.x, me = (int)threadIdx.x;
     const int nlanes = 8 * d.n;
@@ -903,6 +906,7 @@ constexpr int FLOW_THREADS = 128;
 constexpr int FLOW_NBR = 16;          // partners of a particle
 constexpr int FLOW_CHUNK = 16;        // sub-steps between two partner searches
 constexpr double FLOW_SLACK = 0.02;   // radii
+constexpr int COOP_MIN_SUBSTEPS = 3;
 // In more than one block, fewer sub-steps than this run the two-phase form: a
 // partner search and commit cost 12-20 us (2000 / 10,000 particles: 29 / 46 us
 // for one sub-step against 18 / 21, 29 / 48 for two against 26 / 40, 31 / 50
@@ -1030,6 +1034,7 @@ __device__ __noinline__ void flow_two_phase(const DemArgs &A, int parity, int ns
 // MB: resident blocks per SM the registers are cut for (2: none spilled; 3: 168 registers, some spills)
 template <bool WRAP, int LPP, int MB>
 __global__ void __launch_bounds__(FLOW_THREADS, MB) k_dem_flow(const __grid_constant__ FlowArgs f) {
+    grid_dependency();
     constexpr int GPB = FLOW_THREADS / LPP;          // particles per block
     constexpr int K = FLOW_NBR / LPP;                // pairs per lane
     constexpr int NW = (6 + LPP - 1) / LPP;          // walls per lane
@@ -1610,14 +1615,14 @@ int lbdem_dem_launches_last(void) { return g_dem_launches; }
 // 87 us (two-phase 210).
 struct FlowForm {
     int lanes;
-    const void *kern[2];   // without / with periodic images
+    void (*kern[2])(const FlowArgs);   // without / with periodic images
 };
 constexpr int FLOW_FORMS = 4;
 static const FlowForm flow_forms[FLOW_FORMS] = {
-    {8, {(const void *)k_dem_flow<false, 8, 2>, (const void *)k_dem_flow<true, 8, 2>}},
-    {4, {(const void *)k_dem_flow<false, 4, 2>, (const void *)k_dem_flow<true, 4, 2>}},
-    {4, {(const void *)k_dem_flow<false, 4, 3>, (const void *)k_dem_flow<true, 4, 3>}},
-    {2, {(const void *)k_dem_flow<false, 2, 3>, (const void *)k_dem_flow<true, 2, 3>}},
+    {8, {k_dem_flow<false, 8, 2>, k_dem_flow<true, 8, 2>}},
+    {4, {k_dem_flow<false, 4, 2>, k_dem_flow<true, 4, 2>}},
+    {4, {k_dem_flow<false, 4, 3>, k_dem_flow<true, 4, 3>}},
+    {2, {k_dem_flow<false, 2, 3>, k_dem_flow<true, 2, 3>}},
 };
 
 // The form for D's particles (index), or -1 where none applies.  Periodic axes
@@ -1633,7 +1638,7 @@ static int flow_form(const lbdem_dem *D, int dev, int *blocks) {
         *blocks = nb;
         if (nb == 1) return l;
         int coop = 0, nsm = 0, per_sm = 0;
-        if (!D->sync || !coop_residency(dev, 2 + 2 * l + wrap, flow_forms[l].kern[wrap], coop, nsm, per_sm) || !coop)
+        if (!D->sync || !coop_residency(dev, 2 + 2 * l + wrap, (const void *)flow_forms[l].kern[wrap], coop, nsm, per_sm) || !coop)
             return -1;
         if (nb <= per_sm * nsm) return l;
     }
@@ -1659,11 +1664,11 @@ int lbdem_dem_substeps_flow(lbdem_dem *D, int32_t nsub, void *work, void *stream
     f.work = static_cast<unsigned char *>(work);
     f.nsub = nsub;
     cudaStream_t st = (cudaStream_t)stream;
-    const void *kern = flow_forms[form].kern[D->wrap_pairs != 0];
+    auto *kern = flow_forms[form].kern[D->wrap_pairs != 0];
     void *args[] = {&f};
     const int threads = nb > 1 ? FLOW_THREADS : (flow_forms[form].lanes * D->n + 31) / 32 * 32;
-    const cudaError_t e = nb > 1 ? cudaLaunchCooperativeKernel(kern, dim3(nb), dim3(threads), args, 0, st)
-                                 : cudaLaunchKernel(kern, dim3(1), dim3(threads), args, 0, st);
+    const cudaError_t e = nb > 1 ? cudaLaunchCooperativeKernel((const void *)kern, dim3(nb), dim3(threads), args, 0, st)
+                                 : launch_chained(kern, dim3(1), dim3(threads), 0, st, f);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return lbdem_dem_substeps(D, nsub, stream);
@@ -1699,8 +1704,7 @@ int lbdem_dem_substeps(lbdem_dem *D, int32_t nsub, void *stream) {
     const bool one_block = !mode && 8ll * D->n <= 512;
     if (one_block && 8ll * D->n <= 128) {
         A.parity = D->parity;
-        if (wrap) k_dem_block<true><<<1, 128, 0, st>>>(A, (int)nsub);
-        else k_dem_block<false><<<1, 128, 0, st>>>(A, (int)nsub);
+        launch_chained(wrap ? k_dem_block<true> : k_dem_block<false>, dim3(1), dim3(128), 0, st, A, (int)nsub);
         D->parity ^= (nsub & 1);
         g_dem_launches = 1;
         return check_launch("dem_substeps (one block)");
@@ -1738,8 +1742,10 @@ int lbdem_dem_substeps(lbdem_dem *D, int32_t nsub, void *stream) {
         }
     }
     // default: one cooperative launch for all sub-steps when one resident wave
-    // covers the contact lanes ("split" forces two launches per sub-step)
-    if (D->sync && !(mode && strcmp(mode, "split") == 0)) {
+    // covers the contact lanes ("split" forces two launches per sub-step), from
+    // three sub-steps on: below, its barrier reset and launch cost more than two
+    // chained launches per sub-step
+    if (D->sync && !(mode && strcmp(mode, "split") == 0) && (mode || nsub >= COOP_MIN_SUBSTEPS)) {
         int dev = 0, coop = 0, nsm = 0, per_sm = 0;
         cudaGetDevice(&dev);
         if (coop_residency(dev, wrap, (const void *)kcoop, coop, nsm, per_sm) && coop && per_sm > 0) {
@@ -1770,9 +1776,8 @@ int lbdem_dem_substeps(lbdem_dem *D, int32_t nsub, void *stream) {
     const int nb_con64 = (int)((8ll * D->n + 63) / 64), nb_int64 = 2 * nb_int;
     for (int s = 0; s < nsub; ++s) {
         A.parity = D->parity;
-        if (wrap) k_contacts<true><<<nb_con64, 64, 0, st>>>(A);
-        else k_contacts<false><<<nb_con64, 64, 0, st>>>(A);
-        k_integrate<<<nb_int64, 64, 0, st>>>(A);
+        launch_chained(wrap ? k_contacts<true> : k_contacts<false>, dim3(nb_con64), dim3(64), 0, st, A);
+        launch_chained(k_integrate, dim3(nb_int64), dim3(64), 0, st, A);
         D->parity ^= 1;
     }
     g_dem_launches = 2 * nsub;

@@ -131,6 +131,7 @@ __device__ __forceinline__ void particle_table(const MapArgs &a, int g) {
 // compile to the single original sphere.
 template <bool WRAP>
 __global__ void __launch_bounds__(128) k_map_clear(const MapArgs a) {
+    grid_dependency();
     const int g = blockIdx.x;
     bool clear = a.have_prev != 0;
     if (a.disp_limit > 0.0 && a.have_prev && threadIdx.x == 0 && blockIdx.y == 0) {
@@ -269,6 +270,7 @@ constexpr int MAP_MIN_BLOCKS = 10;      // per SM (48 registers, 20 KB of shared
 // diameter 8 from 145 to 116 us and 2000 of diameter 10 from 44 to 41.
 template <bool WRAP>
 __global__ void __launch_bounds__(MAP_THREADS, WRAP ? 8 : MAP_MIN_BLOCKS) k_map_scatter(const MapArgs a) {
+    grid_dependency();
     __shared__ float4 s_off[MAP_CHUNK];   // (xc - i, yc - j, zc - k) in FP32; w = global cell index
     __shared__ int s_amb[MAP_CHUNK];      // partial cells needing the exact recount (index into s_off)
     __shared__ int s_n, s_na;
@@ -655,11 +657,11 @@ extern "C" int lbdem_psc_map(const lbdem_lattice *L, lbdem_psc *P, const lbdem_g
     const bool clear_pass = a.have_prev || a.moved != nullptr || a.disp_limit > 0.0;
     a.table_in_scatter = !clear_pass;
     if (a.wrap[0] || a.wrap[1] || a.wrap[2]) {
-        if (clear_pass) k_map_clear<true><<<sgrid, 128, 0, st>>>(a);
-        k_map_scatter<true><<<sgrid, MAP_THREADS, 0, st>>>(a);
+        if (clear_pass) launch_chained(k_map_clear<true>, sgrid, dim3(128), 0, st, a);
+        launch_chained(k_map_scatter<true>, sgrid, dim3(MAP_THREADS), 0, st, a);
     } else {
-        if (clear_pass) k_map_clear<false><<<sgrid, 128, 0, st>>>(a);
-        k_map_scatter<false><<<sgrid, MAP_THREADS, 0, st>>>(a);
+        if (clear_pass) launch_chained(k_map_clear<false>, sgrid, dim3(128), 0, st, a);
+        launch_chained(k_map_scatter<false>, sgrid, dim3(MAP_THREADS), 0, st, a);
     }
     P->have_prev = 1;
     return check_launch("psc_map");

@@ -263,6 +263,7 @@ class DEMSolver:
         d.status = N.ptr(self.status)
         d.sync = N.ptr(self.sync)
         self._binned = False
+        self._moving = None            # any particle not frozen (None: not looked at since the flags changed)
 
     # ---------------------------------------------------------------- restart
     _STATE_EXTRA = ("cf_j", "cf_active", "cfn", "cf_add", "cf_shear", "cf_pos", "cf_force", "wcf_active", "wcf_shear",
@@ -287,6 +288,7 @@ class DEMSolver:
             getattr(self, k).copy_(d["contact." + k])
         self.status.zero_()
         self._binned = False   # the broad-phase lists are rebuilt from the restored positions
+        self._moving = None
 
     def save_state(self, path):
         torch.save(self.state_dict(), path)
@@ -343,6 +345,14 @@ class DEMSolver:
     def _touched(self, name):
         if name in ("position", "radius"):
             self._binned = False
+        if name == "freeze":
+            self._moving = None
+
+    def any_moving(self) -> bool:
+        """Whether some particle is not frozen (read from the device when the flags were written since)."""
+        if self._moving is None:
+            self._moving = bool((self._t["freeze"] == 0).any())
+        return self._moving
 
     # ---------------------------------------------------------------- stepping
     def _ensure_binned(self):

@@ -91,7 +91,6 @@ class PSCLattice3D(LatticeEngine):
         self._pipeline_probe = None       # (sequential, pipelined) ms per step of that measurement
         self._near = None
         self._side = None
-        self._clear_stream = None
         if solid_fraction == "smooth":
             self._eps = torch.zeros(nc, dtype=torch.float32, device=dev)
             self._map_scratch = torch.zeros(nc, dtype=torch.int64, device=dev)
@@ -242,35 +241,36 @@ class PSCLattice3D(LatticeEngine):
         self._run_pipelined(n, sub_cycles)
 
     def _run_sequential(self, n: int, sub_cycles: int):
-        """step() n times.  Where particles move (so the map cannot be reused),
-        the owner keys of each step's map but the last are cleared on a second
-        stream beside the DEM sub-steps (lbdem_psc_map_clear) instead of by the
-        next map: the step kernel is their last reader, and the next map then
-        claims on clear keys."""
-        early = (n > 1 and self.dem.n > 0 and self.solid_fraction == "exact"
-                 and bool((self.dem._t["freeze"] == 0).any()))
-        if not early:
-            for _ in range(n):
-                self.step(sub_cycles)
+        """step() n times, issued by one native call (lbdem_psc_run).  Where
+        particles move (so the map cannot be reused), each step but the last
+        clears the owner keys that it reads, and the next map claims on clear
+        keys."""
+        d = self.dem
+        native = (d.n > 0 and self.solid_fraction == "exact" and self._initialized and d.contact_model is not None
+                  and not getattr(self, "_kernel_events", None))
+        # a pending stress output or a collide() not streamed yet belongs to an ordinary step
+        while n > 0 and (not native or self._stress_pending or self._collided is not None):
+            self.step(sub_cycles)
+            n -= 1
+        if n <= 0:
             return
-        S = torch.cuda.current_stream()
-        if self._clear_stream is None:
-            self._clear_stream = torch.cuda.Stream()   # default priority: the DEM's blocks are not held back
-        D = self._clear_stream
-        lat, psc, grains = C.byref(self._lat), C.byref(self._psc), C.byref(self._grains)
-        for k in range(n):
-            self.collide()
-            self.stream()
-            stepped = torch.cuda.Event()
-            stepped.record(S)
-            self.dem.run_substeps(sub_cycles)
-            if k < n - 1:
-                with torch.cuda.stream(D):
-                    D.wait_event(stepped)
-                    N.call("lbdem_psc_map_clear", lat, psc, grains, D.cuda_stream)
-                    cleared = torch.cuda.Event()
-                    cleared.record(D)
-                S.wait_event(cleared)
+        self._sync_inputs()
+        if sub_cycles > 0:
+            d._ensure_binned()
+        self._psc.map_reuse = int(self._mapped_epoch == self._links_epoch)
+        done, launches = C.c_int32(0), C.c_int32(0)
+        try:
+            N.call("lbdem_psc_run", C.byref(self._lat), C.byref(self._psc), C.byref(self._grains), C.byref(d._d),
+                   N.ptr(d.flow), n, int(sub_cycles), self._cur, int(self._cur_kind == "fpc"),
+                   int(n > 1 and not self.has_open_boundaries and d.any_moving()),
+                   C.byref(done), C.byref(launches), N.stream_handle())
+        finally:
+            N.count_launches(launches.value)
+            self._mapped_epoch = self._links_epoch
+            if done.value > 0:
+                self._cur = (self._cur + done.value) % 2
+                self._cur_kind, self._collided = "fpc", None
+            self._invalidate_views()
 
     def _side_stream(self):
         if self._side is None:
