@@ -175,18 +175,30 @@ def count_launches(n: int):
     _launches[0] += n
 
 
+# what a call's launches depend on, beyond KERNELS_PER_CALL
+_KIND = {"lbdem_psc_map": 1, "lbdem_dem_substeps": 2, "lbdem_dem_substeps_flow": 2, "lbdem_psc_step_phase": 3,
+         **{name: 4 for name in _BOUNDARY_CALLS}}
+_fns = {}      # name -> (function, its _KIND, kernels per call)
+
+
+def _bind(name: str):
+    entry = _fns[name] = (getattr(load(), name), _KIND.get(name, 0), KERNELS_PER_CALL.get(name, 0))
+    return entry
+
+
 def call(name: str, *args):
-    pre = _map_launches(args[1]) if name == "lbdem_psc_map" else None
-    rc = getattr(load(), name)(*args)
-    if pre is not None:
-        _launches[0] += pre
-    else:
-        _launches[0] += (load().lbdem_dem_launches_last() if name.startswith("lbdem_dem_substeps")
-                         else KERNELS_PER_CALL.get(name, 0))
-    if name == "lbdem_psc_step_phase" and args[8]:
-        _launches[0] += 1     # a launch sized from an estimate is followed by the one that takes the rest
-    if name in _BOUNDARY_CALLS or (name == "lbdem_psc_step_phase" and args[5] == 2):
-        _launches[0] += _boundary_phases(args[0])
+    fn, kind, kernels = _fns.get(name) or _bind(name)
+    if kind == 1:
+        kernels = _map_launches(args[1])
+    rc = fn(*args)
+    if kind == 2:
+        kernels = _lib.lbdem_dem_launches_last()
+    elif kind >= 3:
+        if kind == 3:
+            kernels += args[8] != 0     # a launch sized from an estimate is followed by the one that takes the rest
+        if kind == 4 or args[5] == 2:
+            kernels += _boundary_phases(args[0])
+    _launches[0] += kernels
     if rc != LBDEM_OK:
         msg = load().lbdem_last_error().decode(errors="replace")
         raise LbdemError(f"{name} failed (code {rc}): {msg}")
@@ -198,9 +210,24 @@ def ptr(t):
     return None if t is None else t.data_ptr()
 
 
-def stream_handle():
+_stream = None
+
+
+def _bind_stream():
+    global _stream
     import torch
-    return torch.cuda.current_stream().cuda_stream
+    raw, dev = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    if raw is None or dev is None:
+        _stream = lambda: torch.cuda.current_stream().cuda_stream   # noqa: E731
+    else:
+        torch.cuda.current_stream()    # (initialises the device)
+        _stream = lambda: raw(dev())   # noqa: E731  (a tenth of the cost of a Stream object)
+
+
+def stream_handle():
+    if _stream is None:
+        _bind_stream()
+    return _stream()
 
 
 def require_cuda():

@@ -231,6 +231,7 @@ class DEMSolver:
 
         d = N.Dem()
         self._d = d
+        self._d_ref, self._flow_ptr = C.byref(d), N.ptr(self.flow)   # (both belong to this object, for its life)
         d.n, d.maxc = n, maxc
         d.dt = cfg.dt
         d.g[:] = [float(v) for v in cfg.gravity]
@@ -367,7 +368,7 @@ class DEMSolver:
         if self.n == 0 or nsub <= 0:
             return
         self._ensure_binned()
-        N.call("lbdem_dem_substeps_flow", C.byref(self._d), int(nsub), N.ptr(self.flow), N.stream_handle())
+        N.call("lbdem_dem_substeps_flow", self._d_ref, int(nsub), self._flow_ptr, N.stream_handle())
 
     def run_simulation(self):
         """One DEM time step (demsolver.py:848-862)."""

@@ -439,11 +439,10 @@ class LatticeEngine:
         sel = [slice(None)] * 3
         sel[dim] = int(position)
         fl = (ct[tuple(sel)] & CellType.FLUID) != 0
-        n = int(fl.sum().item())
-        if n == 0:
-            return np.zeros(3)
-        out = torch.stack([st[k][tuple(sel)][fl].double().sum() for k in (3, 4, 5)]) / n
-        return out.cpu().numpy()
+        # the three sums and the count in one device read
+        sums = torch.where(fl, st[3:6][(slice(None), *sel)].double(), 0.0).sum((1, 2))
+        *sums, n = torch.cat([sums, fl.sum(dtype=torch.float64)[None]]).cpu().numpy()
+        return np.array(sums) / n if n > 0 else np.zeros(3)
 
     # ------------------------------------------------------------ restart
     def state_dict(self):
