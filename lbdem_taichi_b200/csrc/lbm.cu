@@ -543,8 +543,13 @@ __device__ __forceinline__ void reduce_forces(const StepArgs &a, CellForce c) {
 // ---------------------------------------------------------------------------
 // fused step, one cell per thread
 // ---------------------------------------------------------------------------
-constexpr int ONE_THREADS = 256;
-constexpr int ONE_MIN_BLOCKS = 4;
+// Two warps a block, 16 blocks per SM (64 registers): a warp with owned cells
+// runs about twice as long as one without, and a block holds all its registers
+// until its last warp ends.  Of blocks of 8, 4 and 2 warps a packed bed of 362 x 122 x 122
+// cells takes 210, 195 and 192 us, the 128^3 bed 59.1, 56.5 and 55.6, the 512
+// x 256 x 256 channel 1004, 993 and 994, the 256^3 suspension 487, 483 and 484.
+constexpr int ONE_THREADS = 64;
+constexpr int ONE_MIN_BLOCKS = 16;
 
 // Moving walls (VEL_LADD neighbours, lbm_solver3d.py:222-225): the bounced
 // population gains 2 w_q rho (c_q . u_wall)/cs^2, rho being the cell's density
@@ -754,8 +759,9 @@ __global__ void __launch_bounds__(ONE_THREADS, ONE_MIN_BLOCKS) k_psc_step(const 
 // The list entries beyond those a listed launch of k_psc_step covered (from
 // a.lbase), a warp per entry, striding by the grid's warps: a launch sized
 // from an earlier step's list length leaves none or a few for this one.
+constexpr int LIST_REST_THREADS = 256;
 template <typename T, int SMAG, int LAGM>
-__global__ void __launch_bounds__(ONE_THREADS) k_psc_step_listed_rest(const StepArgs a) {
+__global__ void __launch_bounds__(LIST_REST_THREADS) k_psc_step_listed_rest(const StepArgs a) {
     const uint32_t n = *a.bcount;
     const uint32_t stride = gridDim.x * (blockDim.x >> 5);
     for (uint32_t w = a.lbase + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < n; w += stride) {
@@ -1983,23 +1989,23 @@ static void set_periods(StepArgs &a, const lbdem_psc *P) {
     a.wrap_any = a.per_x > 0.f || a.per_y > 0.f || a.per_z > 0.f;
 }
 
-// Blocks of w x-blocks (32 w threads) by `by` rows, w by = 8 warps: the split
-// of 8 that leaves the fewest warps past the row's end and the last row, wider
-// ones first.  Idle warps hold their registers until their block ends: 362 x
-// 122 x 122 cells (12 x-blocks a row) in blocks of 8 x-blocks left 4 of 16
-// warps idle and took 0.291 ms, in blocks of 4 x 2 0.212 ms.
-static void step_geometry(const lbdem_lattice *L, dim3 &grid, dim3 &block) {
+// Blocks of w x-blocks (32 w threads) by rows, `warps` in all: the split that
+// leaves the fewest warps past the row's end and the last row, wider ones
+// first.  Idle warps hold their registers until their block ends: 362 x 122 x
+// 122 cells (12 x-blocks a row) in blocks of 8 x-blocks left 4 of 16 warps idle
+// and took 0.291 ms, in blocks of 4 x 2 0.212 ms.
+static void step_geometry(const lbdem_lattice *L, dim3 &grid, dim3 &block, unsigned warps = 8) {
     const unsigned nb = (unsigned)(L->nx + 31) / 32, ny = (unsigned)L->ny;
     unsigned w = 0, best = 0;
-    for (unsigned c = 8; c >= 1; c >>= 1) {
-        const unsigned rows = 8 / c, cols = (nb + c - 1) / c;
-        const unsigned warps = cols * c * ((ny + rows - 1) / rows * rows);
-        if (w == 0 || warps < best) {
+    for (unsigned c = warps; c >= 1; c >>= 1) {
+        const unsigned rows = warps / c, cols = (nb + c - 1) / c;
+        const unsigned total = cols * c * ((ny + rows - 1) / rows * rows);
+        if (w == 0 || total < best) {
             w = c;
-            best = warps;
+            best = total;
         }
     }
-    const unsigned rows = std::min(8 / w, ny);
+    const unsigned rows = std::min(warps / w, ny);
     block = dim3(32 * w, rows, 1);
     grid = dim3((nb + w - 1) / w, (ny + rows - 1) / rows, (unsigned)L->nz);
 }
@@ -2206,7 +2212,7 @@ static int launch_step(const lbdem_lattice *L, const lbdem_psc *P, const lbdem_g
         a.stress_out = L->stress;
     }
     dim3 grid, block;
-    step_geometry(L, grid, block);
+    step_geometry(L, grid, block, ONE_THREADS / 32);
     // FP16 lagged state exists under FP32 storage only (fill_args checks)
     constexpr int LAG_H = sizeof(T) == 4 ? LAG_HALF : LAG_STORE;
 #define LBDEM_STEP_CASE(G_, S_)                                                          \
@@ -2319,7 +2325,7 @@ static int launch_step_phase(const lbdem_lattice *L, const lbdem_psc *P, const l
         if (sized) {                                                                      \
             StepArgs r = a;                                                               \
             r.lbase = grid.x * wpb;                                                       \
-            k_psc_step_listed_rest<T, S_, M_><<<nsm, ONE_THREADS, 0, st>>>(r);            \
+            k_psc_step_listed_rest<T, S_, M_><<<nsm, LIST_REST_THREADS, 0, st>>>(r);            \
         }                                                                                 \
         if (phase == 2) launch_boundary<T, S_, BND_GATHER>(L, a, st);                     \
     } while (0)
