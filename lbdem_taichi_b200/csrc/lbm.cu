@@ -2032,19 +2032,30 @@ static PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
 
 // Which form of the gathered full-lattice step runs: 0 per-thread gathers
 // (k_psc_step), 1 row-staged one cell per thread, 2 row-staged two cells per
-// thread.  By default the row-staged forms for 16-bit storage (two cells per
-// thread where Nx is even) and k_psc_step for FP32 (the row-staged FP32 step
-// fits only two CTAs per SM in shared memory and measured 30 % slower);
+// thread.  The pair kernel has the fewer instructions, but three CTAs of one
+// row each per SM (shared memory), so it pays only where a row fills its CTA
+// (8 x-blocks, keys and links by bulk copy), there are rows enough to keep the
+// CTAs turning, and particles' cells make the step long on arithmetic.
+// FP16, us, gathers / pairs (B200; dense suspension unless noted): 256^3
+// 350 / 331, 256x128^2 90 / 85, 240x128^2 89 / 85, 256x96^2 52.5 / 51.5;
+// against 256x64^2 24.5 / 26, 256x40^2 10.5 / 11.8, 226x128^2 (plain loads)
+// 89 / 101, 192x128^2 69 / 79, 128^3 47 / 67, 64x128^2 24 / 62, 256^3 without
+// solid cells 323 / 370.  The one-cell row form lies between the two or above
+// both (224x128^2 79 / 82, 203x97x118 56 / 62), and for FP32 it fits only two
+// CTAs per SM and measured 30 % slower: it is not chosen.
 // LBDEM_STEP_KERNEL=simt, =rows or =rows2 in the environment at the call
 // selects one form for every storage (=rows2 falls back to =rows where it
 // does not apply).
+constexpr int PAIRS_MIN_ROWS = 8192;
 template <typename T>
-static int step_kernel_form() {
+static int step_kernel_form(const StepArgs &a) {
     const char *e = getenv("LBDEM_STEP_KERNEL");
     if (e && strcmp(e, "simt") == 0) return 0;
     if (e && strcmp(e, "rows") == 0) return 1;
     if (e && strcmp(e, "rows2") == 0) return 2;
-    return sizeof(T) == 2 ? 2 : 0;
+    const bool pairs = sizeof(T) == 2 && a.nb == 8u && a.nx % 4 == 0 && a.key != nullptr &&
+                       (int64_t)a.ny * a.nz >= PAIRS_MIN_ROWS;
+    return pairs ? 2 : 0;
 }
 
 template <typename T> constexpr CUtensorMapDataType tmap_type();
@@ -2217,7 +2228,7 @@ static int launch_step(const lbdem_lattice *L, const lbdem_psc *P, const lbdem_g
     constexpr int LAG_H = sizeof(T) == 4 ? LAG_HALF : LAG_STORE;
 #define LBDEM_STEP_CASE(G_, S_)                                                          \
     do {                                                                                 \
-        const int form_ = step_kernel_form<T>();                                         \
+        const int form_ = step_kernel_form<T>(a);                                        \
         if (G_ && !a.stress_out && form_ > 0) {                                          \
             int rc_ = ROWS_NOT_APPLICABLE;                                               \
             if (form_ == 2)                                                              \
