@@ -38,7 +38,8 @@
  *  lbdem_psc_decode       <- PSCLattice3D fields id/volfrac/weight/velsolid
  *                            src/lbdem/psclattice3d.py:45-52
  *  lbdem_dem_bin,
- *  lbdem_dem_substeps     <- DEMSolver.run_simulation     src/dem3d/demsolver/demsolver.py:848-862
+ *  lbdem_dem_substeps,
+ *  lbdem_dem_substeps_flow <- DEMSolver.run_simulation    src/dem3d/demsolver/demsolver.py:848-862
  *                            (BPCD bpcd.py:67-152, resolve :638-740,
  *                             resolve_wall :809-838, update :514-636,
  *                             hertz.py:45-153, linear.py:43-152)
@@ -302,9 +303,11 @@ int lbdem_psc_map_clear(const lbdem_lattice *L, lbdem_psc *P, const lbdem_grains
  * collide them, one cell per thread or -- 16-bit storage, even Nx, an even
  * number of x-blocks -- two x-adjacent cells per thread in f32x2 arithmetic
  * (its force sums group the cells differently: the same forces to FP32
- * rounding).  Defaults: two cells per thread where it applies, else one, for
- * 16-bit storage; per-thread gathers for FP32.  LBDEM_STEP_KERNEL=simt, =rows
- * or =rows2 in the environment selects one form for every storage. */
+ * rounding).  Defaults: two cells per thread for 16-bit storage where rows fill
+ * their thread block (225 to 256 cells, a multiple of 4), there are at least
+ * 8192 rows and particles are mapped; else per-thread gathers.
+ * LBDEM_STEP_KERNEL=simt, =rows or =rows2 in the environment selects one form
+ * for every storage. */
 int lbdem_psc_step_f32(const lbdem_lattice *L, const lbdem_psc *P, const lbdem_grains *G, int32_t src,
                        int32_t dst, int32_t gather, void *stream);
 int lbdem_psc_step_f16(const lbdem_lattice *L, const lbdem_psc *P, const lbdem_grains *G, int32_t src,
@@ -399,15 +402,16 @@ int lbdem_psc_force_adjoint(const lbdem_lattice *L, const lbdem_psc *P, const lb
 
 int lbdem_dem_bin(lbdem_dem *D, void *stream);
 
-/* Kernels launched by the calling thread's last lbdem_dem_substeps (1 for the
- * single-launch form, 2 per sub-step for the split form); for launch counts. */
+/* Kernels launched by the calling thread's last lbdem_dem_substeps or
+ * lbdem_dem_substeps_flow (1 for the single-launch forms, 2 per sub-step for
+ * the split form); for launch counts. */
 int lbdem_dem_launches_last(void);
 /* nsub DEM sub-steps on the stream, in one of these forms (same contact sets
  * and states; only the order of the atomic force sums differs):
  *   n <= 16:  one 128-thread block, block barriers between the phases;
  *   n <= 64:  one 512-thread block (cluster launch), block barriers;
- *   larger, with D->sync (2 words of device memory) and all contact lanes
- *            in one resident wave: one cooperative launch, bounded grid
+ *   larger, three or more sub-steps, with D->sync (2 words of device memory)
+ *            and all contact lanes in one resident wave: one cooperative launch, bounded grid
  *            barriers (LBDEM_ST_WAIT_TIMEOUT if one gives up);
  *   otherwise two launches per sub-step (contacts, integration) in 64-thread
  *            blocks, which also share the GPU with a step on another stream. */
@@ -420,8 +424,8 @@ int lbdem_dem_substeps(lbdem_dem *D, int32_t nsub, void *stream);
  * work: LBDEM_DEM_FLOW_BYTES(n) of 256-byte aligned device memory, zeroed once
  * by the caller and kept by it between calls, for one solver; D->sync must be
  * zeroed once too.  Where the form does not apply (a short periodic axis, more
- * particles than one resident wave holds, a single sub-step of many particles,
- * no workspace, LBDEM_DEM_KERNELS set in the environment) this is
+ * particles than one resident wave holds, one or two sub-steps of many
+ * particles, no workspace, LBDEM_DEM_KERNELS set in the environment) this is
  * lbdem_dem_substeps. */
 #define LBDEM_DEM_FLOW_BYTES(n) (256 + 512 * (size_t)(n))
 int lbdem_dem_substeps_flow(lbdem_dem *D, int32_t nsub, void *work, void *stream);

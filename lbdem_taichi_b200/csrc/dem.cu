@@ -8,11 +8,14 @@
 // the reference's hash (checked on the host).
 //
 // Cells keep fixed-capacity particle lists filled by the binning atomics, so
-// no scan is needed.  Per sub-step two launches: k_contacts (eight lanes per
-// particle: candidate pairs j > i with contact history owned by i, and the six
-// walls; forces go to accumulators) and k_integrate (accumulated + body +
-// fluid force, improved Verlet, quaternion update, contact-list compaction,
-// binning of the new positions into the other half of the counts).
+// no scan is needed.  A sub-step has a contact phase (eight lanes per particle:
+// candidate pairs j > i with contact history owned by i, and the six walls;
+// forces go to accumulators) and an integration (accumulated + body + fluid
+// force, improved Verlet, quaternion update, contact-list compaction, binning
+// of the new positions into the other half of the counts).  Many sub-steps run
+// as one launch: k_dem_flow with a workspace (a particle waits for the
+// particles it can touch), else one block, one cluster or a cooperative grid;
+// otherwise two launches per sub-step, k_contacts and k_integrate.
 // FP64 throughout; compiled with -fmad=false to follow the reference's
 // operation order (and the FP64 oracle) closely.
 #include <math.h>
@@ -789,8 +792,8 @@ __global__ void __launch_bounds__(128) k_dem_block(const __grid_constant__ DemAr
 }
 
 // ---------------------------------------------------------------------------
-// All sub-steps of one call in ONE cooperative launch (the default): every
-// block of the grid is resident (cudaLaunchCooperativeKernel), the contact
+// All sub-steps of one call in ONE cooperative launch (without a workspace, and
+// k_dem_flow's fallback): every block of the grid is resident (cudaLaunchCooperativeKernel), the contact
 // lanes and the particles are grid-strided, and the two phases of each
 // sub-step are separated by a grid barrier.  The barrier is an arrival counter
 // in caller-owned memory (zeroed before each launch); its wait is bounded:
@@ -1743,8 +1746,10 @@ int lbdem_dem_substeps(lbdem_dem *D, int32_t nsub, void *stream) {
     }
     // default: one cooperative launch for all sub-steps when one resident wave
     // covers the contact lanes ("split" forces two launches per sub-step), from
-    // three sub-steps on: below, its barrier reset and launch cost more than two
-    // chained launches per sub-step
+    // three sub-steps on.  On the GPU alone two chained launches per sub-step are
+    // the shorter (2000 particles, 1-4 sub-steps: 15, 25, 33, 43 us against 18,
+    // 27, 37, 47; 150 particles 13, 22, 32, 39 against 18, 27, 35, 43), but each
+    // takes the host 2-3 us to issue, which a longer call does not hide
     if (D->sync && !(mode && strcmp(mode, "split") == 0) && (mode || nsub >= COOP_MIN_SUBSTEPS)) {
         int dev = 0, coop = 0, nsm = 0, per_sm = 0;
         cudaGetDevice(&dev);
