@@ -996,6 +996,12 @@ __global__ void __launch_bounds__(ROW_THREADS + 32, ROW_MIN_BLOCKS) k_psc_step_r
 // Stores are pairs too.  Warps whose 64 cells include wall, moving-wall,
 // open-boundary or skipped cells, or that use the smooth solid fraction, run
 // the one-cell step for each of their two cells instead.
+// What bounds it: latency at 128 registers, 12 consumer warps per SM (60 % of
+// the issue slots, 85 % of the copy rate on its DRAM bytes; 256^3 FP16 dense
+// suspension 328 us).  Other splits of the same register file: one CTA of 15,
+// 14 or 12 consumer warps with 1, 2 or 4 producers 457, 346, 331 us (a thread
+// needs about 1 us to issue a row's 22 copies), no producer and four CTAs 420,
+// cp.async pipelines of 16 warps 371.
 template <typename T> struct Pair16;
 template <> struct Pair16<__half> {
     __device__ __forceinline__ static float2 widen(uint32_t w) {
