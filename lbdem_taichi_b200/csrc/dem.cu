@@ -897,8 +897,8 @@ __global__ void __launch_bounds__(128, 1) k_dem_coop(const __grid_constant__ Dem
 //   commit  after a grid barrier: state, contact slots and broad-phase lists.
 // Nothing is written before the commit, so a chunk whose assumptions fail -- a
 // particle moved farther than m, more than FLOW_NBR partners, a full contact
-// list, a particle leaving the grid -- is done by the two-phase form instead,
-// in the same launch.
+// list, a particle leaving the grid or outside a periodic face -- is done by the
+// two-phase form instead, in the same launch.
 // 10 sub-steps, against the two-phase form (B200): 2000 spheres of a 256^3
 // suspension, a fifth of them in contact, 45 us (106); one sphere 16 us (60);
 // others at flow_forms.  What bounds it now: FP64 latency of an isolated
@@ -1110,6 +1110,10 @@ __global__ void __launch_bounds__(FLOW_THREADS, MB) k_dem_flow(const __grid_cons
                 n0[a] = max(0, min(d.gdim[a] - 2, (int)floor((x + reach) * icell + 1e-9)) - lo0[a] + 1);
                 lo1[a] = n1[a] = code[a] = 0;
                 if (!d.periodic[a]) continue;
+                // The image within reach of the opposite face finds every partner only where both centres lie in
+                // the box: of two across a face, the one outside would list the other and not be listed by it.
+                // (An unwrapped packing's first call, or a frozen particle, which is never wrapped.)
+                bad = bad || !(P.p[a] >= d.dom_min[a] && P.p[a] <= d.dom_max[a]);
                 const double L = d.dom_max[a] - d.dom_min[a];
                 double sh = 0.0;
                 if (P.p[a] < d.dom_min[a] + reach) { sh = L; code[a] = 1 << (2 * a); }

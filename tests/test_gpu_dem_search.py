@@ -1,0 +1,76 @@
+"""What the partner search of the one-launch DEM form assumes, at its edges,
+against two launches per sub-step (which look every pair up afresh): a chunk
+whose particles break an assumption is left to the two-phase form, in the same
+launch, with the same contact sets and states.
+
+States are held to the bounds of tests/test_gpu_dem_flow.py: the forms differ
+in the order of FP64 force sums only.
+"""
+import numpy as np
+import pytest
+
+from tests.gpu_util import HertzContactConfig, make_dem
+
+pytestmark = pytest.mark.gpu
+
+STATE = ("position", "velocity", "force", "omega", "moment")
+
+
+def _solver(L, pos, rad, vel, compat="reference", freeze=None, g=(0, 0, 0)):
+    rad = np.asarray(rad, float)
+    return make_dem((0, L, 0, L, 0, L), 0.05, g, HertzContactConfig(0.3, 0.3, 0.9, 0.9), rad,
+                    2.0 * 4.0 / 3.0 * np.pi * rad ** 3, pos, vel, periodic=(True,) * 3, E=1e3, wall_E=1e3, max_coord=24,
+                    compat=compat, freeze=freeze)
+
+
+def _columns(p, q, side=4, step=4.0):
+    """Copies of the pair (p, q) in the y-z plane: more than one block of particles."""
+    k = step * np.stack(np.meshgrid(np.arange(side), np.arange(side), indexing="ij"), -1).reshape(-1, 2)
+    off = np.concatenate([np.zeros((len(k), 1)), k], 1)
+    return np.concatenate([p + off, q + off])
+
+
+def _run(monkeypatch, mode, dem, nsub):
+    if mode is None:
+        monkeypatch.delenv("LBDEM_DEM_KERNELS", raising=False)
+    else:
+        monkeypatch.setenv("LBDEM_DEM_KERNELS", mode)
+    dem.run_substeps(nsub)
+    monkeypatch.delenv("LBDEM_DEM_KERNELS", raising=False)
+    dem.check_status()
+
+
+def _same(a, b):
+    ca, cb = a.active_contacts(), b.active_contacts()
+    assert set(ca) == set(cb)
+    np.testing.assert_array_equal(a.cfn.cpu().numpy(), b.cfn.cpu().numpy())
+    for q in range(3):
+        x, y = np.array([ca[p][q] for p in sorted(ca)]), np.array([cb[p][q] for p in sorted(cb)])
+        if len(ca):
+            assert np.abs(x - y).max() <= 1e-8 * max(np.abs(y).max(), 1e-12)
+    for k in STATE:
+        x, y = getattr(a.gf, k).to_numpy(), getattr(b.gf, k).to_numpy()
+        assert np.abs(x - y).max() <= (1e-11 if k == "position" else 1e-8 * max(np.abs(y).max(), 1e-12)), k
+
+
+@pytest.mark.parametrize("compat", ["reference", "wrapped"])
+@pytest.mark.parametrize("frozen", [False, True])
+@pytest.mark.parametrize("pairs", [1, 16])
+def test_centres_outside_a_periodic_face(compat, frozen, pairs, monkeypatch):
+    """A centre outside a periodic face (an unwrapped packing, or a frozen
+    particle, which is never wrapped) touches one at the opposite face."""
+    pos = _columns([-0.5, 2.0, 2.0], [17.505, 2.0, 2.0], 1 if pairs == 1 else 4)
+    n = len(pos)
+    rng = np.random.default_rng(7)
+    vel = rng.normal(0, 0.02, (n, 3))
+    freeze = np.zeros(n, np.int32)
+    if frozen:
+        freeze[:n // 2] = 1
+        vel[:n // 2] = 0.0
+    a, b = (_solver(20.0, pos, np.ones(n), vel, compat, freeze) for _ in range(2))
+    for nsub in (4, 17):
+        _run(monkeypatch, "flow", a, nsub)
+        _run(monkeypatch, "split", b, nsub)
+        _same(a, b)
+    if compat == "wrapped":                # (no gravity: only contacts change a velocity)
+        assert np.abs(b.gf.velocity.to_numpy() - vel).max() > 0
