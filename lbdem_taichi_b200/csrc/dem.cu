@@ -1095,9 +1095,10 @@ __global__ void __launch_bounds__(FLOW_THREADS, MB) k_dem_flow(const __grid_cons
                 for (int t = 0; t < 9; ++t) s_I[g][t] = I[t];
             const double T = S * d.dt, mcap = 0.25 * rmax;
             m = flow_budget(d, i, T, P.rad, P.mass);
-            bad = !(m <= mcap);
             // cells that hold every possible partner: centres within reach, of
-            // the particle and of its periodic images
+            // the particle and of its periodic images.  (rmax bounds a partner's
+            // radius; one written above it later would be listed by its owner only.)
+            bad = !(m <= mcap) || P.rad > rmax;
             const double reach = P.rad + rmax + m + mcap;
             // (a superset: a reciprocal and a slack do).  Per axis: n0 cells of
             // the particle from lo0, then n1 of its image from lo1

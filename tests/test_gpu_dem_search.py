@@ -74,3 +74,24 @@ def test_centres_outside_a_periodic_face(compat, frozen, pairs, monkeypatch):
         _same(a, b)
     if compat == "wrapped":                # (no gravity: only contacts change a velocity)
         assert np.abs(b.gf.velocity.to_numpy() - vel).max() > 0
+
+
+@pytest.mark.parametrize("pairs", [1, 16])
+@pytest.mark.parametrize("x", [9.6, 10.2])
+def test_radius_above_the_broad_phase(x, pairs, monkeypatch):
+    """A radius written above the largest one that the broad-phase cells were
+    made for: the small sphere's search box (centre 9.6, cells of 4) ends short
+    of the large one's cell."""
+    pos = _columns([x, 2.0, 2.0], [x + 3.0, 2.0, 2.0], 1 if pairs == 1 else 4, 5.0)
+    n = len(pos)
+    vel = np.zeros((n, 3))
+    vel[n // 2:, 0] = -0.04                # (closes the gap of 0.01 in half of the second call)
+    a, b = (_solver(20.0, pos, np.ones(n), vel) for _ in range(2))
+    for dem in (a, b):
+        rad = np.ones(n)
+        rad[n // 2:] = 1.99
+        dem.gf.radius.from_numpy(rad)
+    for nsub in (4, 17):
+        _run(monkeypatch, "flow", a, nsub)
+        _run(monkeypatch, "split", b, nsub)
+        _same(a, b)
