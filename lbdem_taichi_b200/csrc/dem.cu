@@ -1017,6 +1017,28 @@ __device__ __noinline__ bool flow_proposed(const lbdem_dem &d, double px, double
     return false;
 }
 
+// Whether the broad phase may propose the pair (i, j), i the lower index, at
+// some time while the two move by no more than mi and mj: flow_proposed over
+// those ranges.  On an axis the probed cells of i are the two from
+// floor((h - 1) / 2), h the half cell it lies in.  Near a periodic face, where
+// a particle can wrap or gain an image, the axis counts as proposed.
+template <bool WRAP>
+__device__ __noinline__ bool flow_may_propose(const lbdem_dem &d, int i, int j, double mi, double mj) {
+    for (int a = 0; a < 3; ++a) {
+        const double pi = d.pos[3 * i + a], pj = d.pos[3 * j + a];
+        if (d.periodic[a]) {
+            const double img = WRAP ? d.cell_size : 0.0;
+            if (!(pi - mi >= d.dom_min[a] + img && pi + mi <= d.dom_max[a] - img && pj - mj >= d.dom_min[a] &&
+                  pj + mj <= d.dom_max[a]))
+                continue;
+        }
+        const double h = 0.5 * d.cell_size, x = pi - d.bp_min[a], y = pj - d.bp_min[a];
+        const int lo = ((int)floor((x - mi) / h) - 1) >> 1, hi = ((int)floor((x + mi) / h) - 1) >> 1;
+        if ((int)floor((y + mj) / d.cell_size) < lo || (int)floor((y - mj) / d.cell_size) > hi + 1) return false;
+    }
+    return true;
+}
+
 // the two-phase form over the sub-steps of a chunk whose lists are binned in
 // half `parity` (the body of k_dem_coop)
 template <bool WRAP>
@@ -1211,6 +1233,19 @@ __global__ void __launch_bounds__(FLOW_THREADS, MB) k_dem_flow(const __grid_cons
         for (int o = 1; o < LPP; o <<= 1) matched += __shfl_xor_sync(0xffffffffu, matched, o);
         const int np_most = __reduce_max_sync(0xffffffffu, np);
         const int room = d.maxc - (n_used - matched);     // slots for listed pairs
+        // A slot in use whose partner is not listed: a contact that opened where the broad phase did not propose
+        // the pair, or positions written since.  The two-phase form drops it when the pair is proposed again, so
+        // where that can happen in this chunk it takes over; elsewhere the slot stays, as there.
+        if (act && n_used > matched)
+            for (int o = k; o < min(n_used, d.maxc); o += LPP) {
+                const size_t s = (size_t)i * d.maxc + o;
+                if (!d.cf_active[s]) continue;
+                const int j = d.cf_j[s];
+                bool listed = false;
+                for (int e = 0; e < nn; ++e) listed = listed || s_list[g][e] == j;
+                if (!listed && flow_may_propose<WRAP>(d, i, j, m, flow_budget(d, j, S * d.dt, d.radius[j], d.mass[j])))
+                    bad = true;
+            }
         int wact = 0, wdirty = 0, wnear = 0;
         double wsh[NW][3], wcp[NW][3], wF[NW][3];
         for (int e = 0; e < NW; ++e) {

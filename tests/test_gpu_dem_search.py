@@ -95,3 +95,33 @@ def test_radius_above_the_broad_phase(x, pairs, monkeypatch):
         _run(monkeypatch, "flow", a, nsub)
         _run(monkeypatch, "split", b, nsub)
         _same(a, b)
+
+
+@pytest.mark.parametrize("compat", ["reference", "wrapped"])
+@pytest.mark.parametrize("pairs", [1, 16])
+def test_contacts_opened_by_a_write(pairs, compat, monkeypatch):
+    """A touching pair is moved apart by a write, farther than the search lists
+    but within the probed cells, and back: the contact ends in between, so the
+    second one starts from no shear."""
+    near = _columns([9.0, 2.0, 2.0], [10.995, 2.0, 2.0], 1 if pairs == 1 else 4)
+    far = _columns([9.0, 2.0, 2.0], [11.2, 2.0, 2.0], 1 if pairs == 1 else 4)
+    n = len(near)
+    vel = np.zeros((n, 3))
+    vel[n // 2:, 1] = 2e-3                 # tangential: builds up shear
+    a, b = (_solver(20.0, near, np.ones(n), vel, compat) for _ in range(2))
+    for where, touching in ((None, True), (far, False), (near, True)):
+        for mode, dem in (("flow", a), ("split", b)):
+            if where is not None:
+                dem.gf.position.from_numpy(where)
+                dem.gf.velocity.from_numpy(vel)
+                dem.gf.omega.from_numpy(np.zeros((n, 3)))
+            _run(monkeypatch, mode, dem, 5)
+        assert (len(b.active_contacts()) > 0) == touching
+        _same(a, b)
+    # moved out of every probed cell the slot stays, as the reference's does
+    away = near.copy()
+    away[n // 2:, 0] = 19.5 - 3.0 if pairs == 1 else 3.0
+    for mode, dem in (("flow", a), ("split", b)):
+        dem.gf.position.from_numpy(away)
+        _run(monkeypatch, mode, dem, 5)
+    _same(a, b)
