@@ -42,12 +42,15 @@ struct M3 {
 // even independent ones overlap.  Arguments here are squared lengths, radii,
 // masses and stiffnesses: positive and far from the ends of the range; a root
 // of less than 1e-290 is 0.  Against the library's results over 1e-30 .. 1e30:
-// at most 1 ulp (rcp64) and 1 ulp (sqrt64) apart.
+// at most 1 ulp (rcp64) and 1 ulp (sqrt64) apart.  The reciprocal of an
+// infinity is 0 and that of 0 infinite, as divided (a frozen sphere may have
+// an infinite mass).
 __device__ __forceinline__ double rcp64(double x) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    double a, r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(a) : "d"(x));
+    r = fma(a, fma(-x, a, 1.0), a);
     r = fma(r, fma(-x, r, 1.0), r);
-    return fma(r, fma(-x, r, 1.0), r);
+    return r == r ? r : a;
 }
 __device__ __forceinline__ double rsqrt64(double x) {
     double r;
@@ -172,8 +175,8 @@ __global__ void k_bin(const __grid_constant__ DemArgs A) {
 // of both directions share one root (DemArgs).
 __device__ __forceinline__ void pair_effective(double rad_i, double rad_j, double mass_i, double mass_j, double &Rs,
                                                double &ms) {
-    Rs = rad_i * rad_j * rcp64(rad_i + rad_j);
-    ms = mass_i * mass_j * rcp64(mass_i + mass_j);
+    Rs = rcp64(rcp64(rad_i) + rcp64(rad_j));
+    ms = rcp64(rcp64(mass_i) + rcp64(mass_j));
 }
 __device__ __forceinline__ void contact_force(const DemArgs &A, double Rs, double ms, bool wall, double *shear,
                                               double delta_n, const double *vc, double *F) {
