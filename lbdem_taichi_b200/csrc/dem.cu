@@ -35,16 +35,17 @@ struct M3 {
     double m[3][3];
 };
 
-// Reciprocal and square roots without branches: the hardware's approximation
-// (PTX rcp.approx / rsqrt.approx.ftz.f64, about 22 bits) and two Newton-Raphson
-// steps.  A contact has half a dozen of them, one after another in a chain that
-// nothing hides, and the library forms branch for special values, so that not
-// even independent ones overlap.  Arguments here are squared lengths, radii,
-// masses and stiffnesses: positive and far from the ends of the range; a root
-// of less than 1e-290 is 0.  Against the library's results over 1e-30 .. 1e30:
-// at most 1 ulp (rcp64) and 1 ulp (sqrt64) apart.  The reciprocal of an
-// infinity is 0 and that of 0 infinite, as divided (a frozen sphere may have
-// an infinite mass).
+// Quotients and square roots without branches: the hardware's approximation of
+// the reciprocal or reciprocal root (PTX rcp.approx / rsqrt.approx.ftz.f64,
+// about 22 bits), two Newton-Raphson steps, and Markstein's correction of the
+// quotient or root by its fused remainder ("Computation of elementary functions
+// on the IBM RISC System/6000 processor", 1990).  A contact has half a dozen of
+// them, one after another in a chain that nothing hides, and the library forms
+// branch for special values, so that not even independent ones overlap.
+// Results are those of IEEE division and root for normal arguments whose
+// reciprocal and quotient are normal too (but for cases within 1e-8 ulp of a
+// tie).  A zero or infinite divisor gives what division gives (a frozen sphere
+// may have an infinite mass).
 __device__ __forceinline__ double rcp64(double x) {
     double a, r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(a) : "d"(x));
@@ -52,16 +53,30 @@ __device__ __forceinline__ double rcp64(double x) {
     r = fma(r, fma(-x, r, 1.0), r);
     return r == r ? r : a;
 }
+// a / b given r, 1 / b to an ulp or two
+__device__ __forceinline__ double div64(double a, double b, double r) {
+    const double q = a * r, c = fma(fma(-b, q, a), r, q);
+    return c == c ? c : q;
+}
+__device__ __forceinline__ double div64(double a, double b) { return div64(a, b, rcp64(b)); }
 __device__ __forceinline__ double rsqrt64(double x) {
     double r;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
     r = fma(0.5 * r, fma(-x * r, r, 1.0), r);
     return fma(0.5 * r, fma(-x * r, r, 1.0), r);
 }
-// root of x given r = rsqrt64(x)
+// 1 / sqrt(x) to half an ulp: the last step with the rounding error of x r
+__device__ __forceinline__ double rsqrt64_round(double x) {
+    double r;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    r = fma(0.5 * r, fma(-x * r, r, 1.0), r);
+    const double s = x * r, e = fma(-fma(x, r, -s), r, fma(-s, r, 1.0));
+    return fma(0.5 * r, e, r);
+}
+// root of x given r = rsqrt64(x); of 0 and of infinity, x
 __device__ __forceinline__ double sqrt64(double x, double r) {
-    const double s = x * r;
-    return x > 1e-290 ? fma(0.5 * r, fma(-s, s, x), s) : (x == x ? 0.0 : x);
+    const double s = x * r, c = fma(0.5 * r, fma(-s, s, x), s);
+    return c == c || x < 0.0 ? c : x;
 }
 __device__ __forceinline__ double sqrt64(double x) { return sqrt64(x, rsqrt64(x)); }
 
@@ -111,7 +126,7 @@ __device__ M3 rot_to_x(const double *a) {
         }
     } else {
         const double vx[3][3] = {{0.0, -v[2], v[1]}, {v[2], 0.0, -v[0]}, {-v[1], v[0], 0.0}};
-        const double coef = (1.0 - c) * rcp64(s2);
+        const double coef = div64(1.0 - c, s2);
         for (int r = 0; r < 3; ++r)
             for (int q = 0; q < 3; ++q) {
                 double acc = 0.0;
@@ -216,7 +231,7 @@ __device__ __forceinline__ void contact_force(const DemArgs &A, double Rs, doubl
     F[0] = F0;
     if (tl >= mu * F0 && tl > 0.0) {
         // sliding: the spring is set to the friction limit, F = -kt shear
-        const double ratio = mu * F0 * rcp64(tl);
+        const double ratio = div64(mu * F0, tl);
         shear[1] *= ratio;
         shear[2] *= ratio;
         F[1] = -kt * shear[1];
@@ -245,16 +260,15 @@ struct PState {
 };
 
 // The evaluated part of resolve(i, j) (demsolver.py:676-740) for a touching
-// pair, on values in registers: dv is the minimum-image vector i -> j, il the
-// reciprocal of its length, sh the
-// pair's shear history (updated).  Gives the contact point, the force in the
+// pair, on values in registers: dv is the minimum-image vector i -> j, len its
+// length and il the reciprocal of that, sh the pair's shear history (updated).  Gives the contact point, the force in the
 // contact frame, the lever arms and the force on j (that on i is its exact
 // negative).
 __device__ __forceinline__ void pair_force(const DemArgs &A, const double *pi, const double *vi, const double *wi,
                                            double rad_i, const double *vj, const double *wj, double Rs, double ms,
-                                           const double *dv, double il, double gap, double *sh, double *cp_out,
+                                           const double *dv, double len, double il, double gap, double *sh, double *cp_out,
                                            double *F_out, double *ri, double *rj, double *Fj) {
-    const double a[3] = {dv[0] * il, dv[1] * il, dv[2] * il};
+    const double a[3] = {div64(dv[0], len, il), div64(dv[1], len, il), div64(dv[2], len, il)};
     const M3 R = rot_to_x(a);
     const double delta_n = -gap;
     for (int t = 0; t < 3; ++t) {
@@ -307,8 +321,8 @@ __device__ __forceinline__ void resolve_pair(const DemArgs &A, int i, const PSta
             }
     double dv[3];
     periodic_delta(d, P.p, pj, dv);
-    const double d2 = dot3(dv, dv), il = rsqrt64(d2);
-    const double gap = sqrt64(d2, il) - P.rad - rad_j;
+    const double d2 = dot3(dv, dv), il = rsqrt64(d2), len = sqrt64(d2, il);
+    const double gap = len - P.rad - rad_j;
     bool eval = false;
     if (off >= 0) {
         if (gap < 0) eval = true;
@@ -332,7 +346,7 @@ __device__ __forceinline__ void resolve_pair(const DemArgs &A, int i, const PSta
     double sh[3] = {d.cf_shear[3 * s], d.cf_shear[3 * s + 1], d.cf_shear[3 * s + 2]};
     double ri[3], rj[3], Fj[3], Mi[3], Mj[3], Rs, ms;
     pair_effective(P.rad, rad_j, P.mass, mass_j, Rs, ms);
-    pair_force(A, P.p, P.v, P.w, P.rad, vj, wj, Rs, ms, dv, il, gap, sh, d.cf_pos + 3 * s, d.cf_force + 3 * s, ri,
+    pair_force(A, P.p, P.v, P.w, P.rad, vj, wj, Rs, ms, dv, len, il, gap, sh, d.cf_pos + 3 * s, d.cf_force + 3 * s, ri,
                rj, Fj);
     const double Fi[3] = {-Fj[0], -Fj[1], -Fj[2]};
     cross3(ri, Fi, Mi);
@@ -575,7 +589,10 @@ __device__ __forceinline__ void quat_update(double dt, double q[4], const double
     const double dq2 = +0.5 * (q[3] * w[0] + q[0] * w[1] + q[1] * w[2]);
     const double dq3 = +0.5 * (-q[2] * w[0] + q[1] * w[1] + q[0] * w[2]);
     q[0] += dq0 * dt; q[1] += dq1 * dt; q[2] += dq2 * dt; q[3] += dq3 * dt;
-    const double il = rsqrt64((q[0] * q[0] + q[1] * q[1]) + (q[2] * q[2] + q[3] * q[3]));
+    // within 3.5 half-ulps of q / |q|, as a root and a division would be, which
+    // are the longest chain of a lone particle's sub-step: they took 10 of them
+    // from 13.0 to 14.1 us, this from 12.7 to 13.3
+    const double il = rsqrt64_round((q[0] * q[0] + q[1] * q[1]) + (q[2] * q[2] + q[3] * q[3]));
     for (int t = 0; t < 4; ++t) q[t] *= il;
 }
 
@@ -590,15 +607,15 @@ __device__ __forceinline__ void wrap_position(const lbdem_dem &d, double *p) {
 }
 
 // update (demsolver.py:514-589), translation on values in registers; the
-// position is not wrapped yet.
-__device__ __forceinline__ void translate_update(double dt, int fixed, double imass, const double force[3], double p[3],
-                                                 double v[3], double acc[3]) {
+// position is not wrapped yet.  imass: rcp64(mass).
+__device__ __forceinline__ void translate_update(double dt, int fixed, double mass, double imass, const double force[3],
+                                                 double p[3], double v[3], double acc[3]) {
     if (fixed) {
         for (int t = 0; t < 3; ++t) p[t] += v[t] * dt;
         return;
     }
     double a[3];
-    for (int t = 0; t < 3; ++t) a[t] = force[t] * imass;
+    for (int t = 0; t < 3; ++t) a[t] = div64(force[t], mass, imass);
     for (int t = 0; t < 3; ++t) v[t] += 0.5 * (acc[t] + a[t]) * dt;
     for (int t = 0; t < 3; ++t) p[t] += v[t] * dt + 0.5 * a[t] * (dt * dt);
     for (int t = 0; t < 3; ++t) acc[t] = a[t];
@@ -673,7 +690,7 @@ __device__ void integrate_particle(const lbdem_dem &d, int ncell, int parity, in
             force[t] = f;
         }
         if (!frozen) {
-            translate_update(dt, fixed, rcp64(mass), force, p, v, acc);
+            translate_update(dt, fixed, mass, rcp64(mass), force, p, v, acc);
             wrap_position(d, p);
         }
         for (int t = 0; t < 3; ++t) {
@@ -1315,7 +1332,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, MB) k_dem_flow(const __grid_cons
                         const bool on = (pact >> e) & 1u;
                         held += own && on;
                         const double lr = own ? P.rad : prad[e], hr = own ? prad[e] : P.rad;
-                        const double d2 = dot3(dv, dv), il = rsqrt64(d2), gap = sqrt64(d2, il) - lr - hr;
+                        const double d2 = dot3(dv, dv), il = rsqrt64(d2), len = sqrt64(d2, il), gap = len - lr - hr;
                         // (the reference proposes no pair across a periodic face)
                         const bool proposed = WRAP || img == 0;
                         if (proposed && !(gap < 0) && on &&
@@ -1333,7 +1350,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, MB) k_dem_flow(const __grid_cons
                             fresh += own && !on;
                             pact |= 1u << e;
                             pdirty |= 1u << e;
-                            pair_force(A, lp, lv, lw, lr, hv, hw, pRs[e], pms[e], dv, il, gap, shr, cp, Fc, ri, rj, Fj);
+                            pair_force(A, lp, lv, lw, lr, hv, hw, pRs[e], pms[e], dv, len, il, gap, shr, cp, Fc, ri, rj, Fj);
                             hit = true;
                             for (int t = 0; t < 3; ++t) {
                                 psh[e][t] = shr[t];
@@ -1405,7 +1422,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, MB) k_dem_flow(const __grid_cons
                 }
                 double x[3] = {P.p[0], P.p[1], P.p[2]}, y[3];
                 if (!frozen) {
-                    translate_update(d.dt, fixed, imass, force, P.p, P.v, acc);
+                    translate_update(d.dt, fixed, P.mass, imass, force, P.p, P.v, acc);
                     for (int t = 0; t < 3; ++t) y[t] = P.p[t];
                     wrap_position(d, P.p);
                     double alpha[3];
