@@ -81,10 +81,12 @@ class FrozenBedDrag:
         lat = self.lat
         lat.initialize()
         self._ckpt = {0: lat._f[lat._cur].clone()}
+        own = lat._own_methods()
         for n in range(1, self.n_steps + 1):
             # the bed is frozen: initialize() mapped it for every step; the last one maps again, which resets
-            # the force accumulators that the loss is read from
-            lat.collide() if n == self.n_steps else lat._collide_mapped()
+            # the force accumulators that the loss is read from.  (A collide() that is not the lattice's own is
+            # called for every step.)
+            lat.collide() if n == self.n_steps or not own else lat._collide_mapped()
             lat.stream()
             if n % self.K == 0 and n < self.n_steps:
                 self._ckpt[n] = lat._f[lat._cur].clone()

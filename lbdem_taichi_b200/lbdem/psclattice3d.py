@@ -244,10 +244,12 @@ class PSCLattice3D(LatticeEngine):
         """step() n times, issued by one native call (lbdem_psc_run).  Where
         particles move (so the map cannot be reused), each step but the last
         clears the owner keys that it reads, and the next map claims on clear
-        keys."""
+        keys.  Where one of the methods it stands for is replaced, in a subclass,
+        on the class or on an instance, of the lattice or of the solver, it is
+        step() n times."""
         d = self.dem
         native = (d.n > 0 and self.solid_fraction == "exact" and self._initialized and d.contact_model is not None
-                  and not getattr(self, "_kernel_events", None))
+                  and not getattr(self, "_kernel_events", None) and self._own_methods())
         # a pending stress output or a collide() not streamed yet belongs to an ordinary step
         while n > 0 and (not native or self._stress_pending or self._collided is not None):
             self.step(sub_cycles)
@@ -271,6 +273,11 @@ class PSCLattice3D(LatticeEngine):
                 self._cur = (self._cur + done.value) % 2
                 self._cur_kind, self._collided = "fpc", None
             self._invalidate_views()
+
+    def _own_methods(self) -> bool:
+        """Whether step() and what it calls are this module's and DEMSolver's own."""
+        return all(getattr(getattr(obj, name), "__func__", None) is fn
+                   for obj, fns in ((self, _STEP_METHODS), (self.dem, _DEM_METHODS)) for name, fn in fns.items())
 
     def _side_stream(self):
         if self._side is None:
@@ -366,3 +373,9 @@ class PSCLattice3D(LatticeEngine):
             d.sync = sync
             self._psc.disp_limit = 0.0
         self._invalidate_views()
+
+
+# the methods that lbdem_psc_run stands for, as they are defined
+_STEP_METHODS = {name: getattr(PSCLattice3D, name)
+                 for name in ("step", "collide", "stream", "grains2lattice", "_collide_mapped", "_launch_step")}
+_DEM_METHODS = {"run_substeps": DEMSolver.run_substeps}
