@@ -268,8 +268,8 @@ class PSCLattice3D(LatticeEngine):
                    C.byref(done), C.byref(launches), N.stream_handle())
         finally:
             N.count_launches(launches.value)
-            self._mapped_epoch = self._links_epoch
             if done.value > 0:
+                self._mapped_epoch = self._links_epoch
                 self._cur = (self._cur + done.value) % 2
                 self._cur_kind, self._collided = "fpc", None
             self._invalidate_views()

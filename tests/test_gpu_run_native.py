@@ -62,3 +62,23 @@ def test_drag_run_calls_an_overridden_collide():
     lat.collide = lambda: (calls.append(1), own())
     assert drag.forward() == pytest.approx(loss, rel=1e-9)
     assert len(calls) == 4
+
+
+def test_failed_run_does_not_mark_the_map_current():
+    """A native call that fails before its first map leaves the owner keys as
+    stale as they were: obstacles set before it lose theirs at the next step."""
+    from lbdem_taichi_b200 import _native as N
+    from lbdem_taichi_b200.lbm3d.lbmutils import CellType
+    lat, _ = _system(frozen=True)
+    lat.initialize()
+    lat.run(2, 1, pipeline=False)
+    assert lat._key.cpu().numpy().reshape(36, 40, 48)[:, :, 20:24].any()
+    ct = lat.CT.to_numpy()
+    ct[20:24, :, :] = CellType.OBSTACLE
+    lat.CT.from_numpy(ct)
+    lat._psc.disp_limit = 0.25             # refused by the native loop
+    with pytest.raises(N.LbdemError):
+        lat.run(2, 1, pipeline=False)
+    lat._psc.disp_limit = 0.0
+    lat.run(2, 1, pipeline=False)
+    assert not lat._key.cpu().numpy().reshape(36, 40, 48)[:, :, 20:24].any()
