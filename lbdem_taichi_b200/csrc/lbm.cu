@@ -756,6 +756,18 @@ __global__ void __launch_bounds__(ONE_THREADS, ONE_MIN_BLOCKS) k_psc_step(const 
     step_at<T, GATHER, SMAG, WRAP, STRESS, LAGM>(a, x, y, z);
 }
 
+// The same over blocks of one x-block by eight rows, for narrow lattices whose
+// rows are more than a grid of k_psc_step's blocks (of one row or two) holds in
+// y.  (A row offset for k_psc_step instead, and several launches of it, took
+// the 362 x 122 x 122 bed from 191 to 206 us.)  WRAP's lever arms are the plain
+// ones where no axis has images.
+constexpr int TALL_ROWS = 8;
+template <typename T, bool GATHER, int SMAG, bool STRESS>
+__global__ void __launch_bounds__(32 * TALL_ROWS) k_psc_step_tall(const StepArgs a) {
+    step_at<T, GATHER, SMAG, true, STRESS, LAG_RUNTIME>(a, blockIdx.x * 32 + threadIdx.x,
+                                                        blockIdx.y * TALL_ROWS + threadIdx.y, blockIdx.z);
+}
+
 // The list entries beyond those a listed launch of k_psc_step covered (from
 // a.lbase), a warp per entry, striding by the grid's warps: a launch sized
 // from an earlier step's list length leaves none or a few for this one.
@@ -2249,7 +2261,11 @@ static int launch_step(const lbdem_lattice *L, const lbdem_psc *P, const lbdem_g
                 return check_launch("psc_step");                                         \
             }                                                                            \
         }                                                                                \
-        if (a.stress_out) {                                                              \
+        if (grid.y > 65535u) {                                                           \
+            const dim3 tall(a.nb, (L->ny + TALL_ROWS - 1) / TALL_ROWS, L->nz);           \
+            if (a.stress_out) k_psc_step_tall<T, G_, S_, true><<<tall, dim3(32, TALL_ROWS), 0, st>>>(a);  \
+            else k_psc_step_tall<T, G_, S_, false><<<tall, dim3(32, TALL_ROWS), 0, st>>>(a); \
+        } else if (a.stress_out) {                                                       \
             if (a.wrap_any) k_psc_step<T, G_, S_, true, false, true><<<grid, block, 0, st>>>(a);  \
             else k_psc_step<T, G_, S_, false, false, true><<<grid, block, 0, st>>>(a);           \
         } else if (a.aux16) {                                                            \
