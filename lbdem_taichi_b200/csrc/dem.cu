@@ -18,6 +18,7 @@
 // otherwise two launches per sub-step, k_contacts and k_integrate.
 // FP64 throughout; compiled with -fmad=false to follow the reference's
 // operation order (and the FP64 oracle) closely.
+#include <float.h>
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
@@ -49,14 +50,17 @@ struct M3 {
 __device__ __forceinline__ double rcp64(double x) {
     double a, r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(a) : "d"(x));
+    const bool normal = fabs(a) <= DBL_MAX && a != 0.0;   // (tested beside the steps, not after them)
     r = fma(a, fma(-x, a, 1.0), a);
     r = fma(r, fma(-x, r, 1.0), r);
-    return r == r ? r : a;
+    return normal ? r : a;
 }
 // a / b given r, 1 / b to an ulp or two
 __device__ __forceinline__ double div64(double a, double b, double r) {
-    const double q = a * r, c = fma(fma(-b, q, a), r, q);
-    return c == c ? c : q;
+    const double q = a * r;
+    const bool normal = fabs(q) <= DBL_MAX && r != 0.0;
+    const double c = fma(fma(-b, q, a), r, q);
+    return normal ? c : q;
 }
 __device__ __forceinline__ double div64(double a, double b) { return div64(a, b, rcp64(b)); }
 __device__ __forceinline__ double rsqrt64(double x) {
@@ -76,7 +80,7 @@ __device__ __forceinline__ double rsqrt64_round(double x) {
 // root of x given r = rsqrt64(x); of 0 and of infinity, x
 __device__ __forceinline__ double sqrt64(double x, double r) {
     const double s = x * r, c = fma(0.5 * r, fma(-s, s, x), s);
-    return c == c || x < 0.0 ? c : x;
+    return r == r || x < 0.0 ? c : x;
 }
 __device__ __forceinline__ double sqrt64(double x) { return sqrt64(x, rsqrt64(x)); }
 
