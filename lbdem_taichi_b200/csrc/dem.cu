@@ -939,10 +939,22 @@ constexpr int COOP_MIN_SUBSTEPS = 3;
 // for one sub-step against 18 / 21, 29 / 48 for two against 26 / 40, 31 / 50
 // for three against 35 / 59).
 constexpr int FLOW_MIN_SUBSTEPS = 3;
-constexpr size_t FLOW_HEADER = 256;   // workspace: two failure words (by chunk parity), the epoch, then the packets
+constexpr size_t FLOW_HEADER = 256;   // workspace: two failure words (by chunk parity), the epoch, the hold, then the packets
+// After a chunk that failed, this many chunks at most go to the two-phase form
+// without a search (1, 3, 7, ... while they keep failing; FlowHold): what breaks
+// an assumption lasts -- a frozen particle outside a face, a large sphere amid
+// small ones.  10 sub-steps of beds with such a particle, us, this / every chunk
+// tried first / the cooperative or split form: 2000 spheres 183 / 273 / 181,
+// 6000 309 / 482 / 181, 20,000 599 / 916 / 330 (the forms of 4 and 2 lanes per
+// particle keep their grid for it).
+constexpr unsigned FLOW_HOLD_MAX = 31;
 constexpr int FLOW_STRIDE = 16;       // packets between two slots: no 128-byte line is polled and written for two
 constexpr int FLOW_STATE = 9;         // doubles of a published state: position, velocity, angular velocity
 constexpr int FLOW_TAGS = 2 * FLOW_CHUNK;   // tags of a chunk: no packet of an earlier chunk or call has one of them
+
+struct FlowHold {
+    unsigned left, length;   // chunks left to the two-phase form, and their number in all
+};
 
 struct FlowArgs {
     DemArgs A;
@@ -1064,9 +1076,10 @@ __device__ __noinline__ bool flow_may_propose(const lbdem_dem &d, int i, int j, 
 }
 
 // the two-phase form over the sub-steps of a chunk whose lists are binned in
-// half `parity` (the body of k_dem_coop)
+// half `parity` (the body of k_dem_coop).  Inlined: called, it read every member
+// of A through a generic pointer (2000 spheres 244 us instead of 183).
 template <bool WRAP>
-__device__ __noinline__ void flow_two_phase(const DemArgs &A, int parity, int nsub, unsigned &gen) {
+__device__ __forceinline__ void flow_two_phase(const DemArgs &A, int parity, int nsub, unsigned &gen) {
     const lbdem_dem &d = A.d;
     const int nthr = gridDim.x * blockDim.x, me = blockIdx.x * blockDim.x + threadIdx.x;
     for (int s = 0; s < nsub; ++s) {
@@ -1080,10 +1093,11 @@ __device__ __noinline__ void flow_two_phase(const DemArgs &A, int parity, int ns
     }
 }
 
-// MB: resident blocks per SM the registers are cut for (2: none spilled; 3: 168 registers, some spills)
-template <bool WRAP, int LPP, int MB>
-__global__ void __launch_bounds__(FLOW_THREADS, MB) k_dem_flow(const __grid_constant__ FlowArgs f) {
-    grid_dependency();
+// One chunk: S sub-steps from the lists binned in half `parity`.  True when it
+// failed: nothing was written then, and the lists are binned as before.
+template <bool WRAP, int LPP>
+__device__ __forceinline__ bool flow_chunk(const FlowArgs &f, int parity, int S, int chunk, unsigned long long epoch0,
+                                           unsigned &gen) {
     constexpr int GPB = FLOW_THREADS / LPP;          // particles per block
     constexpr int K = FLOW_NBR / LPP;                // pairs per lane
     constexpr int NW = (6 + LPP - 1) / LPP;          // walls per lane
@@ -1097,467 +1111,489 @@ __global__ void __launch_bounds__(FLOW_THREADS, MB) k_dem_flow(const __grid_cons
     const bool act = i < d.n;
     const double rmax = 0.25 * d.cell_size;
     int *fail_words = reinterpret_cast<int *>(f.work);
-    unsigned long long *epoch = reinterpret_cast<unsigned long long *>(f.work + 16);
-    const unsigned long long epoch0 = *epoch;
-    unsigned gen = 0;
-    int parity = A.parity, done = 0, chunk = 0;
-    while (done < f.nsub) {
-        const int S = min(f.nsub - done, FLOW_CHUNK);
-        const unsigned long long tag0 = epoch0 + (unsigned long long)chunk * FLOW_TAGS;
-        volatile int *fail = fail_words + (chunk & 1);
-        int32_t *count = d.cell_count + (size_t)parity * A.ncell;
-        // ------------------------------------------------------------ build
-        PState P = {};
-        double acc[3] = {}, wd[3] = {}, q[4] = {}, ffl[3] = {}, mfl[3] = {}, af[3] = {}, am[3] = {};
-        double m = 0.0, imass = 0.0, iI = 0.0;
-        int frozen = 1, fixed = 0, n_used = 0;
-        bool bad = false, iso = true;
-        if (k == 0) s_cnt[g] = 0;
-        __syncwarp();
-        if (act) {
-            for (int t = 0; t < 3; ++t) {
-                P.p[t] = d.pos[3 * i + t];
-                P.v[t] = d.vel[3 * i + t];
-                P.w[t] = d.omega[3 * i + t];
-                acc[t] = d.acc[3 * i + t];
-                wd[t] = d.omega_dot[3 * i + t];
-                ffl[t] = d.force_fluid[3 * i + t];
-                mfl[t] = d.moment_fluid[3 * i + t];
-                af[t] = d.acc_force[3 * i + t];
-                am[t] = d.acc_moment[3 * i + t];
+    const unsigned long long tag0 = epoch0 + (unsigned long long)chunk * FLOW_TAGS;
+    volatile int *fail = fail_words + (chunk & 1);
+    int32_t *count = d.cell_count + (size_t)parity * A.ncell;
+    // ------------------------------------------------------------ build
+    PState P = {};
+    double acc[3] = {}, wd[3] = {}, q[4] = {}, ffl[3] = {}, mfl[3] = {}, af[3] = {}, am[3] = {};
+    double m = 0.0, imass = 0.0, iI = 0.0;
+    int frozen = 1, fixed = 0, n_used = 0;
+    bool bad = false, iso = true;
+    if (k == 0) s_cnt[g] = 0;
+    __syncwarp();
+    if (act) {
+        for (int t = 0; t < 3; ++t) {
+            P.p[t] = d.pos[3 * i + t];
+            P.v[t] = d.vel[3 * i + t];
+            P.w[t] = d.omega[3 * i + t];
+            acc[t] = d.acc[3 * i + t];
+            wd[t] = d.omega_dot[3 * i + t];
+            ffl[t] = d.force_fluid[3 * i + t];
+            mfl[t] = d.moment_fluid[3 * i + t];
+            af[t] = d.acc_force[3 * i + t];
+            am[t] = d.acc_moment[3 * i + t];
+        }
+        for (int t = 0; t < 4; ++t) q[t] = d.quat[4 * i + t];
+        P.rad = d.radius[i];
+        P.mass = d.mass[i];
+        frozen = d.freeze[i];
+        fixed = d.fixvel[i];
+        n_used = d.cfn[i];
+        double I[9];
+        for (int t = 0; t < 9; ++t) I[t] = d.inertia[9 * i + t];
+        iso = inertia_iso(I);
+        iI = rcp64(I[0]);
+        imass = rcp64(P.mass);
+        if (!iso && k == 0)
+            for (int t = 0; t < 9; ++t) s_I[g][t] = I[t];
+        const double T = S * d.dt, mcap = 0.25 * rmax;
+        m = flow_budget(d, i, T, P.rad, P.mass);
+        // cells that hold every possible partner: centres within reach, of
+        // the particle and of its periodic images.  (rmax bounds a partner's
+        // radius; one written above it later would be listed by its owner only.)
+        bad = !(m <= mcap) || P.rad > rmax;
+        const double reach = P.rad + rmax + m + mcap;
+        // (a superset: a reciprocal and a slack do).  Per axis: n0 cells of
+        // the particle from lo0, then n1 of its image from lo1
+        const double icell = rcp64(d.cell_size);
+        int lo0[3], lo1[3], n0[3], n1[3], code[3];
+        for (int a = 0; a < 3; ++a) {
+            const double x = P.p[a] - d.bp_min[a];
+            bad = bad || !(x - m > -d.cell_size && x + m < (d.gdim[a] - 1) * d.cell_size);
+            lo0[a] = max(-1, (int)floor((x - reach) * icell - 1e-9));
+            n0[a] = max(0, min(d.gdim[a] - 2, (int)floor((x + reach) * icell + 1e-9)) - lo0[a] + 1);
+            lo1[a] = n1[a] = code[a] = 0;
+            if (!d.periodic[a]) continue;
+            // The image within reach of the opposite face finds every partner only where both centres lie in
+            // the box: of two across a face, the one outside would list the other and not be listed by it.
+            // (An unwrapped packing's first call, or a frozen particle, which is never wrapped.)
+            bad = bad || !(P.p[a] >= d.dom_min[a] && P.p[a] <= d.dom_max[a]);
+            const double L = d.dom_max[a] - d.dom_min[a];
+            double sh = 0.0;
+            if (P.p[a] < d.dom_min[a] + reach) { sh = L; code[a] = 1 << (2 * a); }
+            else if (P.p[a] > d.dom_max[a] - reach) { sh = -L; code[a] = 2 << (2 * a); }
+            if (sh != 0.0) {
+                lo1[a] = max(-1, (int)floor((x + sh - reach) * icell - 1e-9));
+                n1[a] = max(0, min(d.gdim[a] - 2, (int)floor((x + sh + reach) * icell + 1e-9)) - lo1[a] + 1);
             }
-            for (int t = 0; t < 4; ++t) q[t] = d.quat[4 * i + t];
-            P.rad = d.radius[i];
-            P.mass = d.mass[i];
-            frozen = d.freeze[i];
-            fixed = d.fixvel[i];
-            n_used = d.cfn[i];
-            double I[9];
-            for (int t = 0; t < 9; ++t) I[t] = d.inertia[9 * i + t];
-            iso = inertia_iso(I);
-            iI = rcp64(I[0]);
-            imass = rcp64(P.mass);
-            if (!iso && k == 0)
-                for (int t = 0; t < 9; ++t) s_I[g][t] = I[t];
-            const double T = S * d.dt, mcap = 0.25 * rmax;
-            m = flow_budget(d, i, T, P.rad, P.mass);
-            // cells that hold every possible partner: centres within reach, of
-            // the particle and of its periodic images.  (rmax bounds a partner's
-            // radius; one written above it later would be listed by its owner only.)
-            bad = !(m <= mcap) || P.rad > rmax;
-            const double reach = P.rad + rmax + m + mcap;
-            // (a superset: a reciprocal and a slack do).  Per axis: n0 cells of
-            // the particle from lo0, then n1 of its image from lo1
-            const double icell = rcp64(d.cell_size);
-            int lo0[3], lo1[3], n0[3], n1[3], code[3];
-            for (int a = 0; a < 3; ++a) {
-                const double x = P.p[a] - d.bp_min[a];
-                bad = bad || !(x - m > -d.cell_size && x + m < (d.gdim[a] - 1) * d.cell_size);
-                lo0[a] = max(-1, (int)floor((x - reach) * icell - 1e-9));
-                n0[a] = max(0, min(d.gdim[a] - 2, (int)floor((x + reach) * icell + 1e-9)) - lo0[a] + 1);
-                lo1[a] = n1[a] = code[a] = 0;
-                if (!d.periodic[a]) continue;
-                // The image within reach of the opposite face finds every partner only where both centres lie in
-                // the box: of two across a face, the one outside would list the other and not be listed by it.
-                // (An unwrapped packing's first call, or a frozen particle, which is never wrapped.)
-                bad = bad || !(P.p[a] >= d.dom_min[a] && P.p[a] <= d.dom_max[a]);
-                const double L = d.dom_max[a] - d.dom_min[a];
-                double sh = 0.0;
-                if (P.p[a] < d.dom_min[a] + reach) { sh = L; code[a] = 1 << (2 * a); }
-                else if (P.p[a] > d.dom_max[a] - reach) { sh = -L; code[a] = 2 << (2 * a); }
-                if (sh != 0.0) {
-                    lo1[a] = max(-1, (int)floor((x + sh - reach) * icell - 1e-9));
-                    n1[a] = max(0, min(d.gdim[a] - 2, (int)floor((x + sh + reach) * icell + 1e-9)) - lo1[a] + 1);
+        }
+        const int nx = n0[0] + n1[0], nxy = nx * (n0[1] + n1[1]), tot = bad ? 0 : nxy * (n0[2] + n1[2]);
+        const float inx = 1.f / (float)nx, inxy = 1.f / (float)nxy;
+        auto consider = [&](int j, const double *pj, double rj, int image) {
+            double dv[3];
+            if (image_delta(d, P.p, pj, dv) != image) return;        // found through another image
+            const double d2 = dot3(dv, dv), far = P.rad + rj + (m + mcap);
+            if (!(d2 <= far * far)) return;
+            const double near = P.rad + rj + (m + flow_budget(d, j, T, rj, d.mass[j]));
+            if (!(d2 <= near * near)) return;
+            const int at = atomicAdd(&s_cnt[g], 1);
+            if (at < FLOW_NBR) s_list[g][at] = j;
+            else bad = true;
+        };
+        for (int c0 = k; c0 < tot; c0 += 2 * LPP) {
+            // two cells at a time: counts and first two entries in one round
+            // trip, those particles' positions in a second
+            int ci[2], nj[2], image[2], e[2][2];
+            double pj[2][2][3], rj[2][2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int c = c0 + u * LPP;
+                ci[u] = image[u] = nj[u] = e[u][0] = e[u][1] = 0;
+                if (c >= tot) continue;
+                const int iz = (int)(((float)c + 0.5f) * inxy), r = c - iz * nxy;
+                const int iy = (int)(((float)r + 0.5f) * inx), ix = r - iy * nx;
+                const bool bx = ix >= n0[0], by = iy >= n0[1], bz = iz >= n0[2];
+                image[u] = (bx ? code[0] : 0) | (by ? code[1] : 0) | (bz ? code[2] : 0);
+                ci[u] = cell_index(d, bx ? lo1[0] + ix - n0[0] : lo0[0] + ix, by ? lo1[1] + iy - n0[1] : lo0[1] + iy,
+                                   bz ? lo1[2] + iz - n0[2] : lo0[2] + iz);
+                const int32_t *lst = d.cell_list + (size_t)ci[u] * d.cell_cap;
+                nj[u] = count[ci[u]];
+                e[u][0] = lst[0];
+                e[u][1] = d.cell_cap > 1 ? lst[1] : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                bad = bad || nj[u] > d.cell_cap;
+                nj[u] = min(nj[u], d.cell_cap);
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    if (t >= nj[u]) e[u][t] = i;
+                    const int j = e[u][t];
+                    for (int a = 0; a < 3; ++a) pj[u][t][a] = d.pos[3 * j + a];
+                    rj[u][t] = d.radius[j];
                 }
             }
-            const int nx = n0[0] + n1[0], nxy = nx * (n0[1] + n1[1]), tot = bad ? 0 : nxy * (n0[2] + n1[2]);
-            const float inx = 1.f / (float)nx, inxy = 1.f / (float)nxy;
-            auto consider = [&](int j, const double *pj, double rj, int image) {
-                double dv[3];
-                if (image_delta(d, P.p, pj, dv) != image) return;        // found through another image
-                const double d2 = dot3(dv, dv), far = P.rad + rj + (m + mcap);
-                if (!(d2 <= far * far)) return;
-                const double near = P.rad + rj + (m + flow_budget(d, j, T, rj, d.mass[j]));
-                if (!(d2 <= near * near)) return;
-                const int at = atomicAdd(&s_cnt[g], 1);
-                if (at < FLOW_NBR) s_list[g][at] = j;
-                else bad = true;
-            };
-            for (int c0 = k; c0 < tot; c0 += 2 * LPP) {
-                // two cells at a time: counts and first two entries in one round
-                // trip, those particles' positions in a second
-                int ci[2], nj[2], image[2], e[2][2];
-                double pj[2][2][3], rj[2][2];
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int c = c0 + u * LPP;
-                    ci[u] = image[u] = nj[u] = e[u][0] = e[u][1] = 0;
-                    if (c >= tot) continue;
-                    const int iz = (int)(((float)c + 0.5f) * inxy), r = c - iz * nxy;
-                    const int iy = (int)(((float)r + 0.5f) * inx), ix = r - iy * nx;
-                    const bool bx = ix >= n0[0], by = iy >= n0[1], bz = iz >= n0[2];
-                    image[u] = (bx ? code[0] : 0) | (by ? code[1] : 0) | (bz ? code[2] : 0);
-                    ci[u] = cell_index(d, bx ? lo1[0] + ix - n0[0] : lo0[0] + ix, by ? lo1[1] + iy - n0[1] : lo0[1] + iy,
-                                       bz ? lo1[2] + iz - n0[2] : lo0[2] + iz);
-                    const int32_t *lst = d.cell_list + (size_t)ci[u] * d.cell_cap;
-                    nj[u] = count[ci[u]];
-                    e[u][0] = lst[0];
-                    e[u][1] = d.cell_cap > 1 ? lst[1] : 0;
-                }
+            for (int u = 0; u < 2; ++u) {
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    bad = bad || nj[u] > d.cell_cap;
-                    nj[u] = min(nj[u], d.cell_cap);
-#pragma unroll
-                    for (int t = 0; t < 2; ++t) {
-                        if (t >= nj[u]) e[u][t] = i;
-                        const int j = e[u][t];
-                        for (int a = 0; a < 3; ++a) pj[u][t][a] = d.pos[3 * j + a];
-                        rj[u][t] = d.radius[j];
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-#pragma unroll
-                    for (int t = 0; t < 2; ++t)
-                        if (e[u][t] != i) consider(e[u][t], pj[u][t], rj[u][t], image[u]);
-                    for (int t = 2; t < nj[u]; ++t) {
-                        const int j = d.cell_list[(size_t)ci[u] * d.cell_cap + t];
-                        const double p[3] = {d.pos[3 * j], d.pos[3 * j + 1], d.pos[3 * j + 2]};
-                        if (j != i) consider(j, p, d.radius[j], image[u]);
-                    }
+                for (int t = 0; t < 2; ++t)
+                    if (e[u][t] != i) consider(e[u][t], pj[u][t], rj[u][t], image[u]);
+                for (int t = 2; t < nj[u]; ++t) {
+                    const int j = d.cell_list[(size_t)ci[u] * d.cell_cap + t];
+                    const double p[3] = {d.pos[3 * j], d.pos[3 * j + 1], d.pos[3 * j + 2]};
+                    if (j != i) consider(j, p, d.radius[j], image[u]);
                 }
             }
         }
-        __syncwarp();
-        // this lane's pairs: partner, its constants, and the shear history of a
-        // contact that the lower index already lists
-        const int nn = act ? min(s_cnt[g], FLOW_NBR) : 0;
-        int pj[K], pslot[K];                       // partner; slot of the lower index, -1: none yet
-        unsigned pact = 0, pdirty = 0;             // bit e: pair e is in contact / was evaluated
-        double prad[K], pRs[K], pms[K], psh[K][3], pcp[K][3], pF[K][3];
-        int np = 0, matched = 0;
-        for (int e = k; e < nn; e += LPP, ++np) {
-            const int j = s_list[g][e], own = min(i, j), other = max(i, j);
-            pj[np] = j;
-            prad[np] = d.radius[j];
-            pair_effective(P.rad, prad[np], P.mass, d.mass[j], pRs[np], pms[np]);
-            const int no = min(d.cfn[own], d.maxc);
-            int off = -1;
-            for (int o = 0; o < no && off < 0; ++o)
-                if (d.cf_j[(size_t)own * d.maxc + o] == other && d.cf_active[(size_t)own * d.maxc + o]) off = o;
-            pslot[np] = off;
-            for (int t = 0; t < 3; ++t) psh[np][t] = off >= 0 ? d.cf_shear[3 * ((size_t)own * d.maxc + off) + t] : 0.0;
-            if (off >= 0) {
-                pact |= 1u << np;
-                matched += own == i;
-            }
+    }
+    __syncwarp();
+    // this lane's pairs: partner, its constants, and the shear history of a
+    // contact that the lower index already lists
+    const int nn = act ? min(s_cnt[g], FLOW_NBR) : 0;
+    int pj[K], pslot[K];                       // partner; slot of the lower index, -1: none yet
+    unsigned pact = 0, pdirty = 0;             // bit e: pair e is in contact / was evaluated
+    double prad[K], pRs[K], pms[K], psh[K][3], pcp[K][3], pF[K][3];
+    int np = 0, matched = 0;
+    for (int e = k; e < nn; e += LPP, ++np) {
+        const int j = s_list[g][e], own = min(i, j), other = max(i, j);
+        pj[np] = j;
+        prad[np] = d.radius[j];
+        pair_effective(P.rad, prad[np], P.mass, d.mass[j], pRs[np], pms[np]);
+        const int no = min(d.cfn[own], d.maxc);
+        int off = -1;
+        for (int o = 0; o < no && off < 0; ++o)
+            if (d.cf_j[(size_t)own * d.maxc + o] == other && d.cf_active[(size_t)own * d.maxc + o]) off = o;
+        pslot[np] = off;
+        for (int t = 0; t < 3; ++t) psh[np][t] = off >= 0 ? d.cf_shear[3 * ((size_t)own * d.maxc + off) + t] : 0.0;
+        if (off >= 0) {
+            pact |= 1u << np;
+            matched += own == i;
         }
-        __syncwarp();
-        for (int o = 1; o < LPP; o <<= 1) matched += __shfl_xor_sync(0xffffffffu, matched, o);
-        const int np_most = __reduce_max_sync(0xffffffffu, np);
-        const int room = d.maxc - (n_used - matched);     // slots for listed pairs
-        // A slot in use whose partner is not listed: a contact that opened where the broad phase did not propose
-        // the pair, or positions written since.  The two-phase form drops it when the pair is proposed again, so
-        // where that can happen in this chunk it takes over; elsewhere the slot stays, as there.
-        if (act && n_used > matched)
-            for (int o = k; o < min(n_used, d.maxc); o += LPP) {
-                const size_t s = (size_t)i * d.maxc + o;
-                if (!d.cf_active[s]) continue;
-                const int j = d.cf_j[s];
-                bool listed = false;
-                for (int e = 0; e < nn; ++e) listed = listed || s_list[g][e] == j;
-                if (!listed && flow_may_propose<WRAP>(d, i, j, m, flow_budget(d, j, S * d.dt, d.radius[j], d.mass[j])))
-                    bad = true;
-            }
-        int wact = 0, wdirty = 0, wnear = 0;
-        double wsh[NW][3], wcp[NW][3], wF[NW][3];
-        for (int e = 0; e < NW; ++e) {
-            const int w = k + e * LPP;
-            if (!act || w >= 6 || d.wall_periodic[w]) continue;
-            if (d.wcf_active[(size_t)i * 6 + w]) wact |= 1 << e;
-            // walls within the particle's displacement (normals are unit vectors; any other length only widens it)
-            const double *nrm = d.wall_n + 3 * w;
-            const double sep = -(dot3(P.p, nrm) - d.wall_d[w]);
-            if (((wact >> e) & 1) || !(sep > P.rad + m * (fabs(nrm[0]) + fabs(nrm[1]) + fabs(nrm[2])))) wnear |= 1 << e;
-            for (int t = 0; t < 3; ++t) wsh[e][t] = d.wcf_shear[3 * ((size_t)i * 6 + w) + t];
+    }
+    __syncwarp();
+    for (int o = 1; o < LPP; o <<= 1) matched += __shfl_xor_sync(0xffffffffu, matched, o);
+    const int np_most = __reduce_max_sync(0xffffffffu, np);
+    const int room = d.maxc - (n_used - matched);     // slots for listed pairs
+    // A slot in use whose partner is not listed: a contact that opened where the broad phase did not propose
+    // the pair, or positions written since.  The two-phase form drops it when the pair is proposed again, so
+    // where that can happen in this chunk it takes over; elsewhere the slot stays, as there.
+    if (act && n_used > matched)
+        for (int o = k; o < min(n_used, d.maxc); o += LPP) {
+            const size_t s = (size_t)i * d.maxc + o;
+            if (!d.cf_active[s]) continue;
+            const int j = d.cf_j[s];
+            bool listed = false;
+            for (int e = 0; e < nn; ++e) listed = listed || s_list[g][e] == j;
+            if (!listed && flow_may_propose<WRAP>(d, i, j, m, flow_budget(d, j, S * d.dt, d.radius[j], d.mass[j])))
+                bad = true;
         }
-        if (bad) *fail = 1;
-        // half a grid barrier: the lists may be cleared once every block has built
-        __syncthreads();
-        if (threadIdx.x == 0 && gridDim.x > 1) red_release_gpu(d.sync, 1u);
-        ++gen;
-        bool failed;
-        {
-            // -------------------------------------------------------- flow
-            double D[3] = {0.0, 0.0, 0.0}, force[3], moment[3];
-            bool lost = false, late = false;
-            const bool walls = __any_sync(0xffffffffu, wnear != 0);
-            for (int s = 0; s < S; ++s) {
-                double F[3] = {0.0, 0.0, 0.0}, M[3] = {0.0, 0.0, 0.0};
-                int held = 0, fresh = 0;
-                bool hit = false;                         // this lane evaluated a contact
-                for (int e = 0; e < np_most; ++e) {
-                    const bool have = e < np;
-                    const int j = have ? pj[e] : i;
-                    const bool own = i < j;
-                    double o[FLOW_STATE];
-                    if (s == 0) {
-                        if (have)
-                            for (int t = 0; t < 3; ++t) {
-                                o[t] = d.pos[3 * j + t];
-                                o[3 + t] = d.vel[3 * j + t];
-                                o[6 + t] = d.omega[3 * j + t];
-                            }
-                    } else {
-                        // The warp polls as one: a lane spinning by itself leaves the warp split, and every
-                        // later exchange between its lanes then costs hundreds of cycles (a contact between
-                        // two SMs: 14,300 cycles per sub-step with a loop per lane).  Bounded: about 2^20 looks.
-                        bool wait = have && !lost;
-                        for (unsigned it = 0; __any_sync(0xffffffffu, wait); ++it) {
-                            if (wait) {
-                                const int failed = *fail;
-                                wait = !flow_look(flow_packets(f, j, s & 1), tag0 + s, o);
-                                if (wait && (failed || it >= (1u << 20))) {
-                                    late = late || !failed;
-                                    lost = true;          // the chunk has failed: no more waits
-                                    wait = false;
-                                }
-                            }
-                        }
-                    }
-                    if (have && !lost) {
-                        double lp[3], hp[3], dv[3];
+    int wact = 0, wdirty = 0, wnear = 0;
+    double wsh[NW][3], wcp[NW][3], wF[NW][3];
+    for (int e = 0; e < NW; ++e) {
+        const int w = k + e * LPP;
+        if (!act || w >= 6 || d.wall_periodic[w]) continue;
+        if (d.wcf_active[(size_t)i * 6 + w]) wact |= 1 << e;
+        // walls within the particle's displacement (normals are unit vectors; any other length only widens it)
+        const double *nrm = d.wall_n + 3 * w;
+        const double sep = -(dot3(P.p, nrm) - d.wall_d[w]);
+        if (((wact >> e) & 1) || !(sep > P.rad + m * (fabs(nrm[0]) + fabs(nrm[1]) + fabs(nrm[2])))) wnear |= 1 << e;
+        for (int t = 0; t < 3; ++t) wsh[e][t] = d.wcf_shear[3 * ((size_t)i * 6 + w) + t];
+    }
+    if (bad) *fail = 1;
+    // half a grid barrier: the lists may be cleared once every block has built
+    __syncthreads();
+    if (threadIdx.x == 0 && gridDim.x > 1) red_release_gpu(d.sync, 1u);
+    ++gen;
+    bool failed;
+    {
+        // -------------------------------------------------------- flow
+        double D[3] = {0.0, 0.0, 0.0}, force[3], moment[3];
+        bool lost = false, late = false;
+        const bool walls = __any_sync(0xffffffffu, wnear != 0);
+        for (int s = 0; s < S; ++s) {
+            double F[3] = {0.0, 0.0, 0.0}, M[3] = {0.0, 0.0, 0.0};
+            int held = 0, fresh = 0;
+            bool hit = false;                         // this lane evaluated a contact
+            for (int e = 0; e < np_most; ++e) {
+                const bool have = e < np;
+                const int j = have ? pj[e] : i;
+                const bool own = i < j;
+                double o[FLOW_STATE];
+                if (s == 0) {
+                    if (have)
                         for (int t = 0; t < 3; ++t) {
-                            lp[t] = own ? P.p[t] : o[t];
-                            hp[t] = own ? o[t] : P.p[t];
+                            o[t] = d.pos[3 * j + t];
+                            o[3 + t] = d.vel[3 * j + t];
+                            o[6 + t] = d.omega[3 * j + t];
                         }
-                        const int img = image_delta(d, lp, hp, dv);
-                        const bool on = (pact >> e) & 1u;
-                        held += own && on;
-                        const double lr = own ? P.rad : prad[e], hr = own ? prad[e] : P.rad;
-                        const double d2 = dot3(dv, dv), il = rsqrt64(d2), len = sqrt64(d2, il), gap = len - lr - hr;
-                        // (the reference proposes no pair across a periodic face)
-                        const bool proposed = WRAP || img == 0;
-                        if (proposed && !(gap < 0) && on &&
-                            flow_proposed<WRAP>(d, lp[0], lp[1], lp[2], hp[0], hp[1], hp[2]))
-                            pact &= ~(1u << e);
-                        if (proposed && gap < 0) {
-                            double lv[3], lw[3], hv[3], hw[3], shr[3], cp[3], Fc[3], ri[3], rj[3], Fj[3], Ms[3];
-                            for (int t = 0; t < 3; ++t) {
-                                lv[t] = own ? P.v[t] : o[3 + t];
-                                lw[t] = own ? P.w[t] : o[6 + t];
-                                hv[t] = own ? o[3 + t] : P.v[t];
-                                hw[t] = own ? o[6 + t] : P.w[t];
-                                shr[t] = on ? psh[e][t] : 0.0;
-                            }
-                            fresh += own && !on;
-                            pact |= 1u << e;
-                            pdirty |= 1u << e;
-                            pair_force(A, lp, lv, lw, lr, hv, hw, pRs[e], pms[e], dv, len, il, gap, shr, cp, Fc, ri, rj, Fj);
-                            hit = true;
-                            for (int t = 0; t < 3; ++t) {
-                                psh[e][t] = shr[t];
-                                pcp[e][t] = cp[t];
-                                pF[e][t] = Fc[t];
-                                ri[t] = own ? ri[t] : rj[t];
-                                Fj[t] = own ? -Fj[t] : Fj[t];
-                            }
-                            cross3(ri, Fj, Ms);
-                            for (int t = 0; t < 3; ++t) {
-                                F[t] += Fj[t];
-                                M[t] += Ms[t];
+                } else {
+                    // The warp polls as one: a lane spinning by itself leaves the warp split, and every
+                    // later exchange between its lanes then costs hundreds of cycles (a contact between
+                    // two SMs: 14,300 cycles per sub-step with a loop per lane).  Bounded: about 2^20 looks.
+                    bool wait = have && !lost;
+                    for (unsigned it = 0; __any_sync(0xffffffffu, wait); ++it) {
+                        if (wait) {
+                            const int failed = *fail;
+                            wait = !flow_look(flow_packets(f, j, s & 1), tag0 + s, o);
+                            if (wait && (failed || it >= (1u << 20))) {
+                                late = late || !failed;
+                                lost = true;          // the chunk has failed: no more waits
+                                wait = false;
                             }
                         }
                     }
-                    __syncwarp();
                 }
-                if (__any_sync(0xffffffffu, fresh != 0)) {
-                    // as the two-phase form counts: slots in use when the sub-step began, plus the new ones
-                    int used = held + fresh, any = fresh;
-                    for (int o = 1; o < LPP; o <<= 1) {
-                        used += __shfl_xor_sync(0xffffffffu, used, o);
-                        any += __shfl_xor_sync(0xffffffffu, any, o);
-                    }
-                    if (any && used > room) *fail = 1;
-                }
-                if (walls) {
-                    for (int e = 0; e < NW; ++e) {
-                        const int w = k + e * LPP;
-                        if (!((wnear >> e) & 1)) continue;
-                        const double sep = -(dot3(P.p, d.wall_n + 3 * w) - d.wall_d[w]);
-                        const bool on = (wact >> e) & 1;
-                        if (on && sep > P.rad) {
-                            wact &= ~(1 << e);
-                            wdirty |= 1 << e;
-                        } else if (on || sep <= P.rad) {
-                            double shr[3], cp[3], Fc[3];
-                            for (int t = 0; t < 3; ++t) shr[t] = on ? wsh[e][t] : 0.0;
-                            wall_force(A, P, w, shr, cp, Fc, F, M);
-                            hit = true;
-                            for (int t = 0; t < 3; ++t) {
-                                wsh[e][t] = shr[t];
-                                wcp[e][t] = cp[t];
-                                wF[e][t] = Fc[t];
-                            }
-                            wact |= 1 << e;
-                            wdirty |= 1 << e;
-                        }
-                    }
-                }
-                __syncwarp();
-                const bool hits = __any_sync(0xffffffffu, hit);
-                if (hits) {
-#pragma unroll
-                    for (int o = 1; o < LPP; o <<= 1)
-                        for (int t = 0; t < 3; ++t) {
-                            F[t] += __shfl_xor_sync(0xffffffffu, F[t], o);
-                            M[t] += __shfl_xor_sync(0xffffffffu, M[t], o);
-                        }
-                }
-                // integration, by every lane of the particle alike (integrate_particle, roles 0 and 1); lanes
-                // without a particle stay with their warp (theirs counts as frozen)
-                for (int t = 0; t < 3; ++t) {
-                    double x = F[t] + (s == 0 ? af[t] : 0.0);
-                    x += P.mass * d.g[t];
-                    x += ffl[t];
-                    force[t] = x;
-                    moment[t] = M[t] + (s == 0 ? am[t] : 0.0) + mfl[t];
-                }
-                double x[3] = {P.p[0], P.p[1], P.p[2]}, y[3];
-                if (!frozen) {
-                    translate_update(d.dt, fixed, P.mass, imass, force, P.p, P.v, acc);
-                    for (int t = 0; t < 3; ++t) y[t] = P.p[t];
-                    wrap_position(d, P.p);
-                    double alpha[3];
-                    if (iso)
-                        for (int t = 0; t < 3; ++t) alpha[t] = moment[t] * iI;
-                    else
-                        angular_general(q, P.w, moment, s_I[g], alpha);
-                    spin_update(d.dt, P.w, wd, alpha);
-                }
-                // publish at once; what no partner waits for comes after
-                if (np_most > 0 && s + 1 < S) {
-                    ulonglong2 *out = flow_packets(f, i, (s + 1) & 1);
-                    const unsigned long long tag = tag0 + s + 1;
-#pragma unroll
+                if (have && !lost) {
+                    double lp[3], hp[3], dv[3];
                     for (int t = 0; t < 3; ++t) {
-                        packet_store(nn > 0 && t % LPP == k, out + t, P.p[t], tag);
-                        packet_store(nn > 0 && (3 + t) % LPP == k, out + 3 + t, P.v[t], tag);
-                        packet_store(nn > 0 && (6 + t) % LPP == k, out + 6 + t, P.w[t], tag);
+                        lp[t] = own ? P.p[t] : o[t];
+                        hp[t] = own ? o[t] : P.p[t];
                     }
-                }
-                if (!frozen) {
-                    quat_update(d.dt, q, P.w);
-                    for (int t = 0; t < 3; ++t) D[t] += y[t] - x[t];
-                    if (y[0] != P.p[0] || y[1] != P.p[1] || y[2] != P.p[2]) {
-                        int c[3];
-                        ref_cell(d, P.p, c);
-                        if (cell_index(d, c[0], c[1], c[2]) < 0) *fail = 1;
-                    }
-                    if (!(dot3(D, D) <= 0.999 * (m * m))) *fail = 1;
-                }
-            }
-            if (late) {
-                atomicOr(d.status, (int)LBDEM_ST_WAIT_TIMEOUT);
-                *fail = 1;
-            }
-            // every block has built by now: clear the lists it read
-            grid_wait(d.sync, gen, d.status);
-            for (int c = me; c < A.ncell; c += nthr) count[c] = 0;
-            if (me == 0) fail_words[(chunk + 1) & 1] = 0;
-            grid_barrier(d.sync, gen, d.status);
-            failed = *fail != 0;
-            if (!failed) {
-                // -------------------------------------------------- commit
-                const size_t base = (size_t)i * d.maxc;
-                int drop = 0, born = 0;
-                if (act) {
-                    if (k == 0) {
+                    const int img = image_delta(d, lp, hp, dv);
+                    const bool on = (pact >> e) & 1u;
+                    held += own && on;
+                    const double lr = own ? P.rad : prad[e], hr = own ? prad[e] : P.rad;
+                    const double d2 = dot3(dv, dv), il = rsqrt64(d2), len = sqrt64(d2, il), gap = len - lr - hr;
+                    // (the reference proposes no pair across a periodic face)
+                    const bool proposed = WRAP || img == 0;
+                    if (proposed && !(gap < 0) && on &&
+                        flow_proposed<WRAP>(d, lp[0], lp[1], lp[2], hp[0], hp[1], hp[2]))
+                        pact &= ~(1u << e);
+                    if (proposed && gap < 0) {
+                        double lv[3], lw[3], hv[3], hw[3], shr[3], cp[3], Fc[3], ri[3], rj[3], Fj[3], Ms[3];
                         for (int t = 0; t < 3; ++t) {
-                            d.pos[3 * i + t] = P.p[t];
-                            d.vel[3 * i + t] = P.v[t];
-                            d.acc[3 * i + t] = acc[t];
-                            d.force[3 * i + t] = force[t];
-                            d.acc_force[3 * i + t] = 0.0;
+                            lv[t] = own ? P.v[t] : o[3 + t];
+                            lw[t] = own ? P.w[t] : o[6 + t];
+                            hv[t] = own ? o[3 + t] : P.v[t];
+                            hw[t] = own ? o[6 + t] : P.w[t];
+                            shr[t] = on ? psh[e][t] : 0.0;
                         }
-                        bin_particle(d, i, d.cell_count + (size_t)(parity ^ (S & 1)) * A.ncell);
-                    }
-                    if (k == LPP - 1) {
+                        fresh += own && !on;
+                        pact |= 1u << e;
+                        pdirty |= 1u << e;
+                        pair_force(A, lp, lv, lw, lr, hv, hw, pRs[e], pms[e], dv, len, il, gap, shr, cp, Fc, ri, rj, Fj);
+                        hit = true;
                         for (int t = 0; t < 3; ++t) {
-                            d.omega[3 * i + t] = P.w[t];
-                            d.omega_dot[3 * i + t] = wd[t];
-                            d.moment[3 * i + t] = moment[t];
-                            d.acc_moment[3 * i + t] = 0.0;
+                            psh[e][t] = shr[t];
+                            pcp[e][t] = cp[t];
+                            pF[e][t] = Fc[t];
+                            ri[t] = own ? ri[t] : rj[t];
+                            Fj[t] = own ? -Fj[t] : Fj[t];
                         }
-                        for (int t = 0; t < 4; ++t) d.quat[4 * i + t] = q[t];
-                    }
-                    for (int e = 0; e < NW; ++e) {
-                        if (!((wdirty >> e) & 1)) continue;
-                        const size_t s = (size_t)i * 6 + k + e * LPP;
-                        d.wcf_active[s] = (wact >> e) & 1;
-                        if ((wact >> e) & 1)
-                            for (int t = 0; t < 3; ++t) {
-                                d.wcf_shear[3 * s + t] = wsh[e][t];
-                                d.wcf_pos[3 * s + t] = wcp[e][t];
-                                d.wcf_force[3 * s + t] = wF[e][t];
-                            }
-                    }
-                    // listed contacts in their slots; dropped ones leave gaps
-                    for (int e = 0; e < np; ++e) {
-                        if (pj[e] < i) continue;
-                        const bool on = (pact >> e) & 1u;
-                        if (pslot[e] < 0) {
-                            born += on;
-                        } else if (!on) {
-                            d.cf_active[base + pslot[e]] = 0;
-                            drop = 1;
-                        } else if ((pdirty >> e) & 1u) {
-                            const size_t s = base + pslot[e];
-                            for (int t = 0; t < 3; ++t) {
-                                d.cf_shear[3 * s + t] = psh[e][t];
-                                d.cf_pos[3 * s + t] = pcp[e][t];
-                                d.cf_force[3 * s + t] = pF[e][t];
-                            }
+                        cross3(ri, Fj, Ms);
+                        for (int t = 0; t < 3; ++t) {
+                            F[t] += Fj[t];
+                            M[t] += Ms[t];
                         }
                     }
                 }
-                // close the gaps, then append the new contacts in lane order
-                int before = 0, all = born, drops = drop;
-#pragma unroll
+                __syncwarp();
+            }
+            if (__any_sync(0xffffffffu, fresh != 0)) {
+                // as the two-phase form counts: slots in use when the sub-step began, plus the new ones
+                int used = held + fresh, any = fresh;
                 for (int o = 1; o < LPP; o <<= 1) {
-                    const int x = __shfl_xor_sync(0xffffffffu, all, o);
-                    before += (k & o) ? x : 0;
-                    all += x;
-                    drops += __shfl_xor_sync(0xffffffffu, drops, o);
+                    used += __shfl_xor_sync(0xffffffffu, used, o);
+                    any += __shfl_xor_sync(0xffffffffu, any, o);
                 }
-                __syncwarp();
-                int kept = n_used;
-                if (act && k == 0 && drops) kept = compact_slots(d, i, n_used);
-                __syncwarp();
-                kept = __shfl_sync(0xffffffffu, kept, 0, LPP);
-                if (act) {
-                    int at = kept + before;
-                    for (int e = 0; e < np; ++e) {
-                        if (pj[e] < i || pslot[e] >= 0 || !((pact >> e) & 1u)) continue;
-                        const size_t s = base + at++;
-                        d.cf_j[s] = pj[e];
-                        d.cf_active[s] = 1;
+                if (any && used > room) *fail = 1;
+            }
+            if (walls) {
+                for (int e = 0; e < NW; ++e) {
+                    const int w = k + e * LPP;
+                    if (!((wnear >> e) & 1)) continue;
+                    const double sep = -(dot3(P.p, d.wall_n + 3 * w) - d.wall_d[w]);
+                    const bool on = (wact >> e) & 1;
+                    if (on && sep > P.rad) {
+                        wact &= ~(1 << e);
+                        wdirty |= 1 << e;
+                    } else if (on || sep <= P.rad) {
+                        double shr[3], cp[3], Fc[3];
+                        for (int t = 0; t < 3; ++t) shr[t] = on ? wsh[e][t] : 0.0;
+                        wall_force(A, P, w, shr, cp, Fc, F, M);
+                        hit = true;
+                        for (int t = 0; t < 3; ++t) {
+                            wsh[e][t] = shr[t];
+                            wcp[e][t] = cp[t];
+                            wF[e][t] = Fc[t];
+                        }
+                        wact |= 1 << e;
+                        wdirty |= 1 << e;
+                    }
+                }
+            }
+            __syncwarp();
+            const bool hits = __any_sync(0xffffffffu, hit);
+            if (hits) {
+#pragma unroll
+                for (int o = 1; o < LPP; o <<= 1)
+                    for (int t = 0; t < 3; ++t) {
+                        F[t] += __shfl_xor_sync(0xffffffffu, F[t], o);
+                        M[t] += __shfl_xor_sync(0xffffffffu, M[t], o);
+                    }
+            }
+            // integration, by every lane of the particle alike (integrate_particle, roles 0 and 1); lanes
+            // without a particle stay with their warp (theirs counts as frozen)
+            for (int t = 0; t < 3; ++t) {
+                double x = F[t] + (s == 0 ? af[t] : 0.0);
+                x += P.mass * d.g[t];
+                x += ffl[t];
+                force[t] = x;
+                moment[t] = M[t] + (s == 0 ? am[t] : 0.0) + mfl[t];
+            }
+            double x[3] = {P.p[0], P.p[1], P.p[2]}, y[3];
+            if (!frozen) {
+                translate_update(d.dt, fixed, P.mass, imass, force, P.p, P.v, acc);
+                for (int t = 0; t < 3; ++t) y[t] = P.p[t];
+                wrap_position(d, P.p);
+                double alpha[3];
+                if (iso)
+                    for (int t = 0; t < 3; ++t) alpha[t] = moment[t] * iI;
+                else
+                    angular_general(q, P.w, moment, s_I[g], alpha);
+                spin_update(d.dt, P.w, wd, alpha);
+            }
+            // publish at once; what no partner waits for comes after
+            if (np_most > 0 && s + 1 < S) {
+                ulonglong2 *out = flow_packets(f, i, (s + 1) & 1);
+                const unsigned long long tag = tag0 + s + 1;
+#pragma unroll
+                for (int t = 0; t < 3; ++t) {
+                    packet_store(nn > 0 && t % LPP == k, out + t, P.p[t], tag);
+                    packet_store(nn > 0 && (3 + t) % LPP == k, out + 3 + t, P.v[t], tag);
+                    packet_store(nn > 0 && (6 + t) % LPP == k, out + 6 + t, P.w[t], tag);
+                }
+            }
+            if (!frozen) {
+                quat_update(d.dt, q, P.w);
+                for (int t = 0; t < 3; ++t) D[t] += y[t] - x[t];
+                if (y[0] != P.p[0] || y[1] != P.p[1] || y[2] != P.p[2]) {
+                    int c[3];
+                    ref_cell(d, P.p, c);
+                    if (cell_index(d, c[0], c[1], c[2]) < 0) *fail = 1;
+                }
+                if (!(dot3(D, D) <= 0.999 * (m * m))) *fail = 1;
+            }
+        }
+        if (late) {
+            atomicOr(d.status, (int)LBDEM_ST_WAIT_TIMEOUT);
+            *fail = 1;
+        }
+        // every block has built by now: clear the lists it read
+        grid_wait(d.sync, gen, d.status);
+        for (int c = me; c < A.ncell; c += nthr) count[c] = 0;
+        if (me == 0) fail_words[(chunk + 1) & 1] = 0;
+        grid_barrier(d.sync, gen, d.status);
+        failed = *fail != 0;
+        if (!failed) {
+            // -------------------------------------------------- commit
+            const size_t base = (size_t)i * d.maxc;
+            int drop = 0, born = 0;
+            if (act) {
+                if (k == 0) {
+                    for (int t = 0; t < 3; ++t) {
+                        d.pos[3 * i + t] = P.p[t];
+                        d.vel[3 * i + t] = P.v[t];
+                        d.acc[3 * i + t] = acc[t];
+                        d.force[3 * i + t] = force[t];
+                        d.acc_force[3 * i + t] = 0.0;
+                    }
+                    bin_particle(d, i, d.cell_count + (size_t)(parity ^ (S & 1)) * A.ncell);
+                }
+                if (k == LPP - 1) {
+                    for (int t = 0; t < 3; ++t) {
+                        d.omega[3 * i + t] = P.w[t];
+                        d.omega_dot[3 * i + t] = wd[t];
+                        d.moment[3 * i + t] = moment[t];
+                        d.acc_moment[3 * i + t] = 0.0;
+                    }
+                    for (int t = 0; t < 4; ++t) d.quat[4 * i + t] = q[t];
+                }
+                for (int e = 0; e < NW; ++e) {
+                    if (!((wdirty >> e) & 1)) continue;
+                    const size_t s = (size_t)i * 6 + k + e * LPP;
+                    d.wcf_active[s] = (wact >> e) & 1;
+                    if ((wact >> e) & 1)
+                        for (int t = 0; t < 3; ++t) {
+                            d.wcf_shear[3 * s + t] = wsh[e][t];
+                            d.wcf_pos[3 * s + t] = wcp[e][t];
+                            d.wcf_force[3 * s + t] = wF[e][t];
+                        }
+                }
+                // listed contacts in their slots; dropped ones leave gaps
+                for (int e = 0; e < np; ++e) {
+                    if (pj[e] < i) continue;
+                    const bool on = (pact >> e) & 1u;
+                    if (pslot[e] < 0) {
+                        born += on;
+                    } else if (!on) {
+                        d.cf_active[base + pslot[e]] = 0;
+                        drop = 1;
+                    } else if ((pdirty >> e) & 1u) {
+                        const size_t s = base + pslot[e];
                         for (int t = 0; t < 3; ++t) {
                             d.cf_shear[3 * s + t] = psh[e][t];
                             d.cf_pos[3 * s + t] = pcp[e][t];
                             d.cf_force[3 * s + t] = pF[e][t];
                         }
                     }
-                    if (k == 0 && (drops || all)) d.cfn[i] = kept + all;
                 }
-            } else {
-                // the lists were cleared: bin the untouched positions again
-                if (act && k == 0) bin_particle(d, i, count);
-                grid_barrier(d.sync, gen, d.status);
             }
+            // close the gaps, then append the new contacts in lane order
+            int before = 0, all = born, drops = drop;
+#pragma unroll
+            for (int o = 1; o < LPP; o <<= 1) {
+                const int x = __shfl_xor_sync(0xffffffffu, all, o);
+                before += (k & o) ? x : 0;
+                all += x;
+                drops += __shfl_xor_sync(0xffffffffu, drops, o);
+            }
+            __syncwarp();
+            int kept = n_used;
+            if (act && k == 0 && drops) kept = compact_slots(d, i, n_used);
+            __syncwarp();
+            kept = __shfl_sync(0xffffffffu, kept, 0, LPP);
+            if (act) {
+                int at = kept + before;
+                for (int e = 0; e < np; ++e) {
+                    if (pj[e] < i || pslot[e] >= 0 || !((pact >> e) & 1u)) continue;
+                    const size_t s = base + at++;
+                    d.cf_j[s] = pj[e];
+                    d.cf_active[s] = 1;
+                    for (int t = 0; t < 3; ++t) {
+                        d.cf_shear[3 * s + t] = psh[e][t];
+                        d.cf_pos[3 * s + t] = pcp[e][t];
+                        d.cf_force[3 * s + t] = pF[e][t];
+                    }
+                }
+                if (k == 0 && (drops || all)) d.cfn[i] = kept + all;
+            }
+        } else {
+            // the lists were cleared: bin the untouched positions again
+            if (act && k == 0) bin_particle(d, i, count);
+            grid_barrier(d.sync, gen, d.status);
         }
-        if (failed) flow_two_phase<WRAP>(A, parity, S, gen);
+    }
+    return failed;
+}
+
+// MB: resident blocks per SM that the registers are cut for (255 at 2, 168 at 3)
+template <bool WRAP, int LPP, int MB>
+__global__ void __launch_bounds__(FLOW_THREADS, MB) k_dem_flow(const __grid_constant__ FlowArgs f) {
+    grid_dependency();
+    const lbdem_dem &d = f.A.d;
+    int *fail_words = reinterpret_cast<int *>(f.work);
+    unsigned long long *epoch = reinterpret_cast<unsigned long long *>(f.work + 16);
+    FlowHold *hold_word = reinterpret_cast<FlowHold *>(f.work + 24);
+    const unsigned long long epoch0 = *epoch;
+    FlowHold hold = *hold_word;               // (the same in every thread throughout)
+    unsigned gen = 0;
+    int parity = f.A.parity, done = 0, chunk = 0;
+    while (done < f.nsub) {
+        const int S = min(f.nsub - done, FLOW_CHUNK);
+        // (expected, so that the two-phase form stays out of the sub-step loop's code: a lone sphere 14.4 us otherwise, 14.1)
+        bool failed = hold.left > 0;
+        if (__builtin_expect(failed, 0)) {
+            --hold.left;
+            // (the next chunk's failure word, as flow_chunk clears it; all have read it: the last use was before a barrier)
+            if (blockIdx.x == 0 && threadIdx.x == 0) fail_words[(chunk + 1) & 1] = 0;
+        } else {
+            failed = flow_chunk<WRAP, LPP>(f, parity, S, chunk, epoch0, gen);
+            hold.length = failed ? min(2 * hold.length + 1, FLOW_HOLD_MAX) : 0;
+            hold.left = hold.length;
+        }
+        if (__builtin_expect(failed, 0)) flow_two_phase<WRAP>(f.A, parity, S, gen);
         parity ^= S & 1;
         done += S;
         ++chunk;
@@ -1567,10 +1603,14 @@ __global__ void __launch_bounds__(FLOW_THREADS, MB) k_dem_flow(const __grid_cons
     if (gridDim.x == 1) {
         __syncthreads();
         if (threadIdx.x < 2) fail_words[threadIdx.x] = 0;
-        if (threadIdx.x == 0) *epoch = epoch0 + (unsigned long long)chunk * FLOW_TAGS;
+        if (threadIdx.x == 0) {
+            *epoch = epoch0 + (unsigned long long)chunk * FLOW_TAGS;
+            *hold_word = hold;
+        }
     } else if (barrier_release(d.sync)) {
         fail_words[0] = fail_words[1] = 0;
         *epoch = epoch0 + (unsigned long long)chunk * FLOW_TAGS;
+        *hold_word = hold;
     }
 }
 

@@ -125,3 +125,39 @@ def test_contacts_opened_by_a_write(pairs, compat, monkeypatch):
         dem.gf.position.from_numpy(away)
         _run(monkeypatch, mode, dem, 5)
     _same(a, b)
+
+
+@pytest.mark.parametrize("side", [2, 6])
+def test_chunks_that_keep_failing(side, monkeypatch):
+    """A particle whose velocity no search covers (frozen, apart from the rest):
+    chunk after chunk fails and the next ones are left to the two-phase form
+    without a search, within a call and across calls; when the cause is gone
+    the searches come back."""
+    pos = 2.0 + 1.995 * np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos[0] = 20.0
+    n = len(pos)
+    rng = np.random.default_rng(4)
+    vel = rng.normal(0, 0.005, (n, 3))
+    vel[0] = (50.0, 0.0, 0.0)
+    freeze = np.zeros(n, np.int32)
+    freeze[0] = 1
+    a, b = (_solver(24.0, pos, np.ones(n), vel, freeze=freeze) for _ in range(2))
+    hold = lambda: a.flow[24:32].cpu().numpy().view(np.uint32)   # chunks left, their number
+    seen = []
+    for nsub in (5, 3, 3, 3, 3, 100, 7):
+        _run(monkeypatch, "flow", a, nsub)
+        _run(monkeypatch, "split", b, nsub)
+        _same(a, b)
+        seen.append(tuple(hold()))
+    # chunks of at most 16: fail | held | fail | held | held | held, fail, 5 of 7 held | held
+    assert seen == [(1, 1), (0, 1), (3, 3), (2, 3), (1, 3), (2, 7), (1, 7)]
+    for dem in (a, b):
+        v = dem.gf.velocity.to_numpy()
+        v[0] = 0.0
+        dem.gf.velocity.from_numpy(v)
+    for nsub in (4, 4, 4):
+        _run(monkeypatch, "flow", a, nsub)
+        _run(monkeypatch, "split", b, nsub)
+        _same(a, b)
+    assert tuple(hold()) == (0, 0)
+    assert not a.flow[:8].any() and not a.sync.any()
