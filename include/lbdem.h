@@ -39,7 +39,8 @@
  *                            src/lbdem/psclattice3d.py:45-52
  *  lbdem_dem_bin,
  *  lbdem_dem_substeps,
- *  lbdem_dem_substeps_flow <- DEMSolver.run_simulation    src/dem3d/demsolver/demsolver.py:848-862
+ *  lbdem_dem_substeps_flow,
+ *  lbdem_dem_flow_bytes   <- DEMSolver.run_simulation    src/dem3d/demsolver/demsolver.py:848-862
  *                            (BPCD bpcd.py:67-152, resolve :638-740,
  *                             resolve_wall :809-838, update :514-636,
  *                             hertz.py:45-153, linear.py:43-152)
@@ -59,6 +60,7 @@
 #ifndef LBDEM_H
 #define LBDEM_H
 
+#include <stddef.h>
 #include <stdint.h>
 
 #ifdef __cplusplus
@@ -429,6 +431,10 @@ int lbdem_dem_substeps(lbdem_dem *D, int32_t nsub, void *stream);
  * lbdem_dem_substeps. */
 #define LBDEM_DEM_FLOW_BYTES(n) (256 + 512 * (size_t)(n))
 int lbdem_dem_substeps_flow(lbdem_dem *D, int32_t nsub, void *work, void *stream);
+
+/* The workspace for D on the current device: LBDEM_DEM_FLOW_BYTES(D->n), or 0
+ * where no call for D would use one (host only; no launch). */
+size_t lbdem_dem_flow_bytes(const lbdem_dem *D);
 
 /* nsteps coupled steps in one call: per step lbdem_psc_map, the fused step
  * (src, then alternating; gather for the first, 1 after) and nsub sub-steps of

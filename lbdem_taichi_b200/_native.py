@@ -21,7 +21,6 @@ ABI_VERSION = 4        # LBDEM_ABI_VERSION of include/lbdem.h
 F32, F16, BF16 = 0, 1, 2
 LINK_FLUID = 1 << 20   # LBDEM_LINK_FLUID: the link mask of every cell of an all-FLUID lattice
 SMAG_OFF, SMAG_REFERENCE, SMAG_LOCAL = 0, 1, 2
-DEM_FLOW_BYTES = (256, 512)   # LBDEM_DEM_FLOW_BYTES: fixed part, per particle
 SUM_BLOCKS = 1184
 SUM_PARTIALS = 4 * SUM_BLOCKS
 
@@ -97,6 +96,7 @@ EXPORTS = {
     "lbdem_dem_bin": ([vp, vp], C.c_int),
     "lbdem_dem_substeps": ([vp, C.c_int32, vp], C.c_int),
     "lbdem_dem_substeps_flow": ([vp, C.c_int32, vp, vp], C.c_int),
+    "lbdem_dem_flow_bytes": ([vp], C.c_size_t),
     "lbdem_global_sums_f64": ([vp, C.c_int32, vp, vp, vp], C.c_int),
     "lbdem_global_sums_f64_noalloc": ([vp, C.c_int32, vp, vp], C.c_int),
     "lbdem_psc_map_smooth": ([vp, vp, vp, vp, vp], C.c_int),

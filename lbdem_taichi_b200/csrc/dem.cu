@@ -1752,6 +1752,12 @@ static int flow_form(const lbdem_dem *D, int dev, int *blocks) {
     return -1;
 }
 
+size_t lbdem_dem_flow_bytes(const lbdem_dem *D) {
+    int dev = 0, nb = 0;
+    if (check_dem(D) || D->n == 0 || cudaGetDevice(&dev) != cudaSuccess || flow_form(D, dev, &nb) < 0) return 0;
+    return LBDEM_DEM_FLOW_BYTES(D->n);
+}
+
 int lbdem_dem_substeps_flow(lbdem_dem *D, int32_t nsub, void *work, void *stream) {
     int rc = check_dem(D);
     if (rc) return rc;

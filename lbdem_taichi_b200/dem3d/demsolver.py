@@ -217,7 +217,6 @@ class DEMSolver:
         self.acc_force = torch.zeros((max(n, 1), 3), **f64)
         self.acc_moment = torch.zeros((max(n, 1), 3), **f64)
         self.sync = torch.zeros(2, **i32)
-        self.flow = torch.zeros(N.DEM_FLOW_BYTES[0] + N.DEM_FLOW_BYTES[1] * n, dtype=torch.uint8, device=DEV)
         # the reference hashes cells into a 2^k table: distinct cells alias when
         # their coordinates agree in the low bits kept by Morton-code mod 2^k
         T = reference_table_size(rmax, dmin, dmax) if n else 1 << 20
@@ -231,7 +230,6 @@ class DEMSolver:
 
         d = N.Dem()
         self._d = d
-        self._d_ref, self._flow_ptr = C.byref(d), N.ptr(self.flow)   # (both belong to this object, for its life)
         d.n, d.maxc = n, maxc
         d.dt = cfg.dt
         d.g[:] = [float(v) for v in cfg.gravity]
@@ -263,6 +261,10 @@ class DEMSolver:
         d.parity = 0
         d.status = N.ptr(self.status)
         d.sync = N.ptr(self.sync)
+        # workspace of the one-launch form, where one of its forms takes these particles
+        need = N.load().lbdem_dem_flow_bytes(C.byref(d))
+        self.flow = torch.zeros(need, dtype=torch.uint8, device=DEV) if need else None
+        self._d_ref, self._flow_ptr = C.byref(d), N.ptr(self.flow)   # (both belong to this object, for its life)
         self._binned = False
         self._moving = None            # any particle not frozen (None: not looked at since the flags changed)
 
