@@ -307,7 +307,9 @@ int lbdem_psc_map_clear(const lbdem_lattice *L, lbdem_psc *P, const lbdem_grains
  * (its force sums group the cells differently: the same forces to FP32
  * rounding).  Defaults: two cells per thread for 16-bit storage where rows fill
  * their thread block (225 to 256 cells, a multiple of 4), there are at least
- * 8192 rows and particles are mapped; else per-thread gathers.
+ * 8192 rows and particles are mapped; without particles two cells or rows of
+ * one where the row is long and the lattice of middle size (step_kernel_form in
+ * csrc/lbm.cu has the lines and their measurements); else per-thread gathers.
  * LBDEM_STEP_KERNEL=simt, =rows or =rows2 in the environment selects one form
  * for every storage. */
 int lbdem_psc_step_f32(const lbdem_lattice *L, const lbdem_psc *P, const lbdem_grains *G, int32_t src,

@@ -2060,20 +2060,46 @@ static PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
 // 89 / 101, 192x128^2 69 / 79, 128^3 47 / 67, 64x128^2 24 / 62, 256^3 without
 // solid cells 323 / 370.  The one-cell row form lies between the two or above
 // both (224x128^2 79 / 82, 203x97x118 56 / 62), and for FP32 it fits only two
-// CTAs per SM and measured 30 % slower: it is not chosen.
+// CTAs per SM and measured 30 % slower: neither takes it.  (Lagged Smagorinsky
+// form; off and local, 256x128^2 79 / 77 and 84 / 83, 128^3 42 / 60 and 44 / 64.)
+// Without particles (no keys, no owned warps) a row costs less and its copies
+// weigh more: pairs from 4096 rows of eight x-blocks or 8192 of six, for as long
+// as the kernel keeps up with DRAM, which its lagged form, with the fifth more
+// to copy, does least, and rows that are not whole 32-byte groups less than
+// others.  FP16 unless noted, gathers / pairs: Smagorinsky off 256x64^2 17.6 /
+// 15.6, 256x128^2 69.4 / 55.0, 192x128^2 54.1 / 49.3, 252x192^2 154 / 171,
+// 256x192^2 152 / 145, 256^3 268 / 279, in BF16 270 / 256; local 256x128^2 77.2
+// / 60.2, 256^3 297 / 270; lagged 256x64^2 21.7 / 18.1, 256x128x96 62.3 / 61.0,
+// 256x128^2 82.8 / 83.1, 256^3 316 / 357, 192^3 136 / 125; all 128^3 37-43 / 42-47.
+// Odd widths and seven x-blocks: one-cell rows where the collision is the
+// longer, gathers / rows: local 251x128^2 78.0 / 72.7, 251x256^2 296 / 279,
+// 224x128^2 68.8 / 66.1; lagged 251x128^2 83.0 / 78.4, 251x256^2 323 / 368; off
+// 251x128^2 70.6 / 69.1, 251x256^2 271 / 273.
 // LBDEM_STEP_KERNEL=simt, =rows or =rows2 in the environment at the call
 // selects one form for every storage (=rows2 falls back to =rows where it
 // does not apply).
 constexpr int PAIRS_MIN_ROWS = 8192;
-template <typename T>
+template <typename T, int SMAG>
 static int step_kernel_form(const StepArgs &a) {
     const char *e = getenv("LBDEM_STEP_KERNEL");
     if (e && strcmp(e, "simt") == 0) return 0;
     if (e && strcmp(e, "rows") == 0) return 1;
     if (e && strcmp(e, "rows2") == 0) return 2;
-    const bool pairs = sizeof(T) == 2 && a.nb == 8u && a.nx % 4 == 0 && a.key != nullptr &&
-                       (int64_t)a.ny * a.nz >= PAIRS_MIN_ROWS;
-    return pairs ? 2 : 0;
+    if (sizeof(T) != 2) return 0;
+    const int64_t rows = (int64_t)a.ny * a.nz;
+    if (a.key != nullptr) return a.nb == 8u && a.nx % 4 == 0 && rows >= PAIRS_MIN_ROWS ? 2 : 0;
+    const bool lagged = SMAG == LBDEM_SMAG_REFERENCE;
+    if (a.nx % 2 == 0 && a.nb == 8u) {
+        if (rows < PAIRS_MIN_ROWS / 2) return 0;
+        if (SMAG == LBDEM_SMAG_LOCAL) return 2;
+        if (lagged) return rows <= 12288 ? 2 : 0;
+        const bool bf16 = Store<T>::kind == LBDEM_BF16;
+        return rows <= 24576 || (a.nx % 16 == 0 && (bf16 || rows <= 36864)) ? 2 : 0;
+    }
+    if (rows < PAIRS_MIN_ROWS) return 0;
+    if (a.nx % 2 == 0 && a.nb == 6u) return 2;
+    if (a.nb == 7u || a.nb == 8u) return SMAG == LBDEM_SMAG_LOCAL || (lagged && rows * a.nb <= 8 * 24576) ? 1 : 0;
+    return 0;
 }
 
 template <typename T> constexpr CUtensorMapDataType tmap_type();
@@ -2246,7 +2272,7 @@ static int launch_step(const lbdem_lattice *L, const lbdem_psc *P, const lbdem_g
     constexpr int LAG_H = sizeof(T) == 4 ? LAG_HALF : LAG_STORE;
 #define LBDEM_STEP_CASE(G_, S_)                                                          \
     do {                                                                                 \
-        const int form_ = step_kernel_form<T>(a);                                        \
+        const int form_ = step_kernel_form<T, S_>(a);                                    \
         if (G_ && !a.stress_out && form_ > 0) {                                          \
             int rc_ = ROWS_NOT_APPLICABLE;                                               \
             if (form_ == 2)                                                              \
