@@ -45,6 +45,7 @@ struct AdjArgs {
     const uint32_t *links;
     const uint32_t *key;
     const float *eps;
+    int zper;                    // cells of a thread along z
 };
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -67,9 +68,13 @@ __device__ __forceinline__ float warp_sum(float v) {
 // which is a third of the arithmetic of summing the 19 directions one by one
 // (the kernel issued instructions all the time at 128 registers and 16 warps
 // per SM: 0.141 ms at 128^3, 3.4 TB/s on its 228 B per cell; so 0.087 ms, 5.5
-// TB/s).  Each thread takes ADJ_Z cells along z, so that the three same-address FP64
-// atomics of dL/dF are a fourth as many.
+// TB/s).  Each thread takes up to ADJ_Z cells along z, so that the three same-address
+// FP64 atomics of dL/dF are a fourth as many -- of lattices that fill the GPU (444
+// resident blocks) many times over; of smaller ones two, or one: 1 / 2 / 4 cells of
+// 32^3 (128 blocks at one) 3.2 / 4.6 / 7.3 us, 48^3 (576) 6.9 / 6.3 / 8.3, 80^3 (3200)
+// 26.5 / 26.3 / 29.2, 128^3 (8192) 87.8 / 84.0 / 85.5, 160^3 (25,600) 173 / 163 / 160.
 constexpr int ADJ_Z = 4;
+static int cells_along_z(int64_t blocks) { return blocks < 444 ? 1 : blocks < 16384 ? ADJ_Z / 2 : ADJ_Z; }
 
 template <bool GATHER, bool SEED>
 __global__ void __launch_bounds__(256, 3) k_psc_adjoint(const AdjArgs a) {
@@ -86,9 +91,9 @@ __global__ void __launch_bounds__(256, 3) k_psc_adjoint(const AdjArgs a) {
     const uint32_t sxp = xslot(xc_ == nx - 1 ? 0u : (uint32_t)(xc_ + 1), QB);
     const float W0 = wq(0), W1 = wq(1), W2 = wq(7);
     float gx = 0.f, gy = 0.f, gz = 0.f;
-    const int z1 = min(nz, ((int)blockIdx.z + 1) * ADJ_Z);
+    const int z1 = min(nz, ((int)blockIdx.z + 1) * a.zper);
 #pragma unroll 1
-    for (int z = blockIdx.z * ADJ_Z; z < z1; ++z) {
+    for (int z = blockIdx.z * a.zper; z < z1; ++z) {
         const uint32_t row = (uint32_t)(z * ny + yc_);
         const uint32_t cell = row * (uint32_t)nx + (uint32_t)xc_;
         const uint32_t r0 = row * rs, own = r0 + sx0;
@@ -333,7 +338,10 @@ extern "C" int lbdem_psc_step_adjoint_f32(const lbdem_lattice *L, const lbdem_ps
     if (bx > 256) bx = 256;
     int by = 256 / bx;
     if (by > L->ny) by = L->ny;
-    const dim3 block(bx, by, 1), grid((L->nx + bx - 1) / bx, (L->ny + by - 1) / by, (L->nz + ADJ_Z - 1) / ADJ_Z);
+    const dim3 block(bx, by, 1);
+    dim3 grid((L->nx + bx - 1) / bx, (L->ny + by - 1) / by, 1);
+    a.zper = cells_along_z((int64_t)grid.x * grid.y * L->nz);
+    grid.z = (L->nz + a.zper - 1) / a.zper;
     cudaStream_t st = (cudaStream_t)stream;
     if (gather) {
         if (seed) k_psc_adjoint<true, true><<<grid, block, 0, st>>>(a);
