@@ -38,3 +38,26 @@ def test_bed(side, images, monkeypatch):
     np.testing.assert_array_equal(a.wcf_active.cpu().numpy(), b.wcf_active.cpu().numpy())
     assert b.wcf_active.any()
     assert not a.flow[24:32].any()                      # no chunk failed
+
+
+@pytest.mark.parametrize("n", [1, 8, 9, 16, 17])
+@pytest.mark.parametrize("nsub", [1, 2, 3, 4])
+def test_short_calls_of_few_particles(n, nsub, monkeypatch):
+    """The default form of short calls, on either side of where one block's
+    two-phase form gives way: 3 sub-steps up to 8 particles, 4 above; more than
+    one block, 3."""
+    from torch.profiler import ProfilerActivity, profile
+    rng = np.random.default_rng(n)
+    pos = 2.0 + 1.995 * np.stack(np.meshgrid(*[np.arange(3)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    vel = rng.normal(0, 0.01, (n, 3))
+    a, b = (make_dem((0, 24, 0, 24, 0, 24), 0.02, (0, 0, -1e-3), HertzContactConfig(0.3, 0.3, 0.9, 0.9), np.ones(n),
+                     np.full(n, 8.0), pos, vel, periodic=(True, True, False), E=1e3, wall_E=1e3) for _ in range(2))
+    for _ in range(3):
+        _run(monkeypatch, None, a, nsub)
+        _run(monkeypatch, "split", b, nsub)
+    _same(a, b)
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        _run(monkeypatch, None, a, nsub)
+    names = {e.name for e in prof.events() if "lbdem::k_" in e.name}
+    flow = nsub >= (3 if n <= 8 or n > 16 else 4)
+    assert any("k_dem_flow" in e for e in names) == flow, names
