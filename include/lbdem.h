@@ -318,6 +318,9 @@ int lbdem_psc_step_f16(const lbdem_lattice *L, const lbdem_psc *P, const lbdem_g
                        int32_t dst, int32_t gather, void *stream);
 int lbdem_psc_step_bf16(const lbdem_lattice *L, const lbdem_psc *P, const lbdem_grains *G, int32_t src,
                         int32_t dst, int32_t gather, void *stream);
+/* The form of the calling thread's last lbdem_psc_step_*: 0 per-thread gathers,
+ * 1 rows staged in shared memory, one cell per thread, 2 two cells per thread. */
+int lbdem_psc_step_form_last(void);
 
 /* Pipelined stepping (no counterpart in the reference: a scheduling of the
  * same step).  The fused step of a coupled lattice only needs the particle map

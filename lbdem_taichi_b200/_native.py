@@ -92,6 +92,7 @@ EXPORTS = {
     "lbdem_psc_step_f16": ([vp, vp, vp, C.c_int32, C.c_int32, C.c_int32, vp], C.c_int),
     "lbdem_psc_step_bf16": ([vp, vp, vp, C.c_int32, C.c_int32, C.c_int32, vp], C.c_int),
     "lbdem_stream_moments": ([vp, C.c_int32, C.c_int32, vp], C.c_int),
+    "lbdem_psc_step_form_last": ([], C.c_int),
     "lbdem_psc_decode": ([vp, vp, vp, vp, vp, vp, vp], C.c_int),
     "lbdem_dem_bin": ([vp, vp], C.c_int),
     "lbdem_dem_substeps": ([vp, C.c_int32, vp], C.c_int),

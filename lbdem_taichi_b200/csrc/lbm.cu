@@ -2079,6 +2079,7 @@ static PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
 // selects one form for every storage (=rows2 falls back to =rows where it
 // does not apply).
 constexpr int PAIRS_MIN_ROWS = 8192;
+static thread_local int g_step_form = 0;   // of the thread's last step (lbdem_psc_step_form_last)
 template <typename T, int SMAG>
 static int step_kernel_form(const StepArgs &a) {
     const char *e = getenv("LBDEM_STEP_KERNEL");
@@ -2275,18 +2276,22 @@ static int launch_step(const lbdem_lattice *L, const lbdem_psc *P, const lbdem_g
         const int form_ = step_kernel_form<T, S_>(a);                                    \
         if (G_ && !a.stress_out && form_ > 0) {                                          \
             int rc_ = ROWS_NOT_APPLICABLE;                                               \
+            g_step_form = 2;                                                             \
             if (form_ == 2)                                                              \
                 rc_ = a.wrap_any ? launch_step_rows<T, S_, true, true>(L, a, st)          \
                                  : launch_step_rows<T, S_, false, true>(L, a, st);        \
-            if (rc_ == ROWS_NOT_APPLICABLE)                                              \
+            if (rc_ == ROWS_NOT_APPLICABLE) {                                            \
+                g_step_form = 1;                                                         \
                 rc_ = a.wrap_any ? launch_step_rows<T, S_, true, false>(L, a, st)         \
                                  : launch_step_rows<T, S_, false, false>(L, a, st);       \
+            }                                                                            \
             if (rc_ != ROWS_NOT_APPLICABLE) {                                            \
                 if (rc_ != LBDEM_OK) return rc_;                                         \
                 launch_boundary<T, S_, BND_GATHER>(L, a, st);                            \
                 return check_launch("psc_step");                                         \
             }                                                                            \
         }                                                                                \
+        g_step_form = 0;                                                                 \
         if (grid.y > 65535u) {                                                           \
             const dim3 tall(a.nb, (L->ny + TALL_ROWS - 1) / TALL_ROWS, L->nz);           \
             if (a.stress_out) k_psc_step_tall<T, G_, S_, true><<<tall, dim3(32, TALL_ROWS), 0, st>>>(a);  \
@@ -2616,6 +2621,8 @@ int lbdem_lattice_init(const lbdem_lattice *L, int32_t buf, void *stream) {
     set_error("unknown storage form %d", L->storage);
     return LBDEM_ERR_ARG;
 }
+
+int lbdem_psc_step_form_last(void) { return g_step_form; }
 
 int lbdem_psc_step_f32(const lbdem_lattice *L, const lbdem_psc *P, const lbdem_grains *G, int32_t src, int32_t dst,
                        int32_t gather, void *stream) {

@@ -46,7 +46,6 @@ def test_short_calls_of_few_particles(n, nsub, monkeypatch):
     """The default form of short calls, on either side of where one block's
     two-phase form gives way: 3 sub-steps up to 8 particles, 4 above; more than
     one block, 3."""
-    from torch.profiler import ProfilerActivity, profile
     rng = np.random.default_rng(n)
     pos = 2.0 + 1.995 * np.stack(np.meshgrid(*[np.arange(3)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
     vel = rng.normal(0, 0.01, (n, 3))
@@ -56,8 +55,5 @@ def test_short_calls_of_few_particles(n, nsub, monkeypatch):
         _run(monkeypatch, None, a, nsub)
         _run(monkeypatch, "split", b, nsub)
     _same(a, b)
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        _run(monkeypatch, None, a, nsub)
-    names = {e.name for e in prof.events() if "lbdem::k_" in e.name}
     flow = nsub >= (3 if n <= 8 or n > 16 else 4)
-    assert any("k_dem_flow" in e for e in names) == flow, names
+    assert (a.flow[16:24].cpu().numpy().view(np.uint64)[0] > 0) == flow   # the one-launch form counts its chunks

@@ -16,8 +16,7 @@ pytestmark = pytest.mark.gpu
 
 
 def _run(mode, shape, storage, smag, wall):
-    from torch.profiler import ProfilerActivity, profile
-
+    from lbdem_taichi_b200 import _native as N
     from lbdem_taichi_b200.lbm3d.lattice import BasicLattice3D
     os.environ["LBDEM_STEP_KERNEL"] = mode
     try:
@@ -30,23 +29,19 @@ def _run(mode, shape, storage, smag, wall):
             lat.CT.from_numpy(ct)
         lat.vel.from_numpy(0.03 * rng.uniform(-1, 1, (*shape, 3)))
         lat.initialize()
-        lat.collide()
-        lat.stream()
-        with profile(activities=[ProfilerActivity.CUDA]) as prof:
-            for _ in range(2):
-                lat.collide()
-                lat.stream()
-            torch.cuda.synchronize()
-        names = {e.name.split("<")[0].split("::")[-1] for e in prof.events() if "k_psc_step" in e.name}
+        for _ in range(3):
+            lat.collide()
+            lat.stream()
+        form = N.load().lbdem_psc_step_form_last()
         out = [lat._f[lat._cur].clone(), lat.rho.to_numpy(), lat.vel.to_numpy()]
         if lat._aux is not None:
             out.append(lat._aux.clone())
-        return names, out
+        return form, out
     finally:
         os.environ.pop("LBDEM_STEP_KERNEL", None)
 
 
-ONE, ROWS, PAIRS = "k_psc_step", "k_psc_step_rows", "k_psc_step_rows2"
+ONE, ROWS, PAIRS = 0, 1, 2
 
 
 @pytest.mark.parametrize("shape,storage,smag,form,wall", [
@@ -61,8 +56,8 @@ ONE, ROWS, PAIRS = "k_psc_step", "k_psc_step_rows", "k_psc_step_rows2"
     ((288, 64, 128), "f16", "local", ONE, None),
 ])
 def test_chosen_form(shape, storage, smag, form, wall):
-    names, got = _run("auto", shape, storage, smag, wall)
-    assert names == {form}
+    ran, got = _run("auto", shape, storage, smag, wall)
+    assert ran == form
     _, want = _run("simt", shape, storage, smag, wall)
     for g, w in zip(got, want):
         g, w = torch.as_tensor(g).double(), torch.as_tensor(w).double()
