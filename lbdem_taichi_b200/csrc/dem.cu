@@ -16,8 +16,11 @@
 // as one launch: k_dem_flow with a workspace (a particle waits for the
 // particles it can touch), else one block, one cluster or a cooperative grid;
 // otherwise two launches per sub-step, k_contacts and k_integrate.
-// FP64 throughout; compiled with -fmad=false to follow the reference's
-// operation order (and the FP64 oracle) closely.
+// FP64 throughout; compiled with -fmad=false, so that every operation rounds as
+// it is written.  The integration follows the reference's order; the contact law
+// is rearranged (one root for both dampings, the transpose of a rotation for its
+// inverse, the spring set by the friction ratio) to the same value within
+// roundings.
 #include <float.h>
 #include <math.h>
 #include <stdlib.h>
@@ -816,13 +819,13 @@ __global__ void __launch_bounds__(128) k_dem_block(const __grid_constant__ DemAr
 }
 
 // ---------------------------------------------------------------------------
-// All sub-steps of one call in ONE cooperative launch (without a workspace, and
-// k_dem_flow's fallback): every block of the grid is resident (cudaLaunchCooperativeKernel), the contact
-// lanes and the particles are grid-strided, and the two phases of each
-// sub-step are separated by a grid barrier.  The barrier is an arrival counter
-// in caller-owned memory (zeroed before each launch); its wait is bounded:
-// after ~0.25 s without progress it sets LBDEM_ST_WAIT_TIMEOUT and continues,
-// so a fault can never hang the GPU.
+// All sub-steps of one call in ONE cooperative launch (without a workspace; also
+// what k_dem_flow falls back to): every block of the grid is resident
+// (cudaLaunchCooperativeKernel), the contact lanes and the particles are
+// grid-strided, and the two phases of each sub-step are separated by a grid
+// barrier.  The barrier is an arrival counter in caller-owned memory, zero at
+// launch; its wait is bounded: after 2^22 looks (some seconds) it sets
+// LBDEM_ST_WAIT_TIMEOUT and continues, so a fault can never hang the GPU.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned *p) {
     unsigned v;
@@ -837,8 +840,9 @@ __device__ __forceinline__ void red_release_gpu(unsigned *p, unsigned v) {
     asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Arrivals count up monotonically in sync[0] (zeroed before each launch): the
-// k-th barrier is passed when the count reaches k * gridDim.x.  One release
+// Arrivals count up monotonically in sync[0] (zero at launch: k_dem_coop's caller
+// zeroes it, k_dem_flow finds it as barrier_release left it): the k-th barrier is
+// passed when the count reaches k * gridDim.x.  One release
 // reduction per block and barrier (after the block barrier, which orders the
 // block's writes of the phase before thread 0, so the release publishes them
 // all), then polling with acquire loads; no reset.
@@ -895,8 +899,9 @@ __global__ void __launch_bounds__(128, 1) k_dem_coop(const __grid_constant__ Dem
 
 // ---------------------------------------------------------------------------
 // All sub-steps of one call in ONE launch without a grid barrier per sub-step:
-// LPP lanes own a particle for the whole call, its state stays in registers,
-// and a particle waits only for the particles it can touch.
+// LPP lanes own a particle for the whole call, its state stays in registers (its
+// pairs' data, indexed at run time, in local memory), and a particle waits only
+// for the particles it can touch.
 //
 // What bounds the sub-steps is latency: two grid barriers and a chain of
 // dependent loads (cell, list, partner, contact slot) per sub-step, for a few
@@ -921,13 +926,15 @@ __global__ void __launch_bounds__(128, 1) k_dem_coop(const __grid_constant__ Dem
 //   commit  after a grid barrier: state, contact slots and broad-phase lists.
 // Nothing is written before the commit, so a chunk whose assumptions fail -- a
 // particle moved farther than m, more than FLOW_NBR partners, a full contact
-// list, a particle leaving the grid or outside a periodic face -- is done by the
-// two-phase form instead, in the same launch.
+// list, a particle leaving the grid or outside a periodic face, a slot in use
+// that the two-phase form may drop -- is done by that form instead, in the same
+// launch.
 // 10 sub-steps, against the two-phase form (B200): 2000 spheres of a 256^3
-// suspension, a fifth of them in contact, 45 us (106); one sphere 16 us (60);
-// others at flow_forms.  What bounds it now: FP64 latency of an isolated
-// particle's sub-step 0.65 us, of one with a contact 1.9 us (half of it the
-// exchange through L2), and 12 us of search, barrier and commit per call.
+// suspension, a fifth of them in contact, 44 us (106); one sphere 14 us alone and
+// 18 between the kernels of a coupled step (60); others at flow_forms.  What
+// bounds it now: FP64 latency of an isolated particle's sub-step 0.7 us, of one
+// with a contact 1.9 us (half of it the exchange through L2), and 7 us (one
+// block) to 12 of search, barrier and commit per call.
 // ---------------------------------------------------------------------------
 constexpr int FLOW_THREADS = 128;
 constexpr int FLOW_NBR = 16;          // partners of a particle
@@ -953,8 +960,8 @@ constexpr size_t FLOW_HEADER = 256;   // workspace: two failure words (by chunk 
 // without a search (1, 3, 7, ... while they keep failing; FlowHold): what breaks
 // an assumption lasts -- a frozen particle outside a face, a large sphere amid
 // small ones.  10 sub-steps of beds with such a particle, us, this / every chunk
-// tried first / the cooperative or split form: 2000 spheres 183 / 273 / 181,
-// 6000 309 / 482 / 181, 20,000 599 / 916 / 330 (the forms of 4 and 2 lanes per
+// tried first / the cooperative or split form: 2000 spheres 186 / 273 / 181,
+// 6000 310 / 482 / 182, 20,000 599 / 916 / 330 (the forms of 4 and 2 lanes per
 // particle keep their grid for it).
 constexpr unsigned FLOW_HOLD_MAX = 31;
 constexpr int FLOW_STRIDE = 16;       // packets between two slots: no 128-byte line is polled and written for two
