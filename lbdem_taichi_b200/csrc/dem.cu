@@ -268,9 +268,9 @@ struct PState {
 
 // The evaluated part of resolve(i, j) (demsolver.py:676-740) for a touching
 // pair, on values in registers: dv is the minimum-image vector i -> j, len its
-// length and il the reciprocal of that, sh the pair's shear history (updated).  Gives the contact point, the force in the
-// contact frame, the lever arms and the force on j (that on i is its exact
-// negative).
+// length and il the reciprocal of that, sh the pair's shear history (updated).
+// Gives the contact point, the force in the contact frame, the lever arms and
+// the force on j (that on i is its exact negative).
 __device__ __forceinline__ void pair_force(const DemArgs &A, const double *pi, const double *vi, const double *wi,
                                            double rad_i, const double *vj, const double *wj, double Rs, double ms,
                                            const double *dv, double len, double il, double gap, double *sh, double *cp_out,
@@ -842,10 +842,10 @@ __device__ __forceinline__ void red_release_gpu(unsigned *p, unsigned v) {
 
 // Arrivals count up monotonically in sync[0] (zero at launch: k_dem_coop's caller
 // zeroes it, k_dem_flow finds it as barrier_release left it): the k-th barrier is
-// passed when the count reaches k * gridDim.x.  One release
-// reduction per block and barrier (after the block barrier, which orders the
-// block's writes of the phase before thread 0, so the release publishes them
-// all), then polling with acquire loads; no reset.
+// passed when the count reaches k * gridDim.x.  One release reduction per block
+// and barrier (after the block barrier, which orders the block's writes of the
+// phase before thread 0, so the release publishes them all), then polling with
+// acquire loads; no reset.
 __device__ __forceinline__ void grid_wait(uint32_t *sync, unsigned gen, int32_t *status) {
     if (gridDim.x > 1 && threadIdx.x == 0) {
         const unsigned target = gen * gridDim.x;
@@ -1623,7 +1623,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, MB) k_dem_flow(const __grid_cons
     int parity = f.A.parity, done = 0, chunk = 0;
     while (done < f.nsub) {
         const int S = min(f.nsub - done, FLOW_CHUNK);
-        // (expected, so that the two-phase form stays out of the sub-step loop's code: a lone sphere 14.4 us otherwise, 14.1)
+        // (expected, so that the two-phase form stays out of the sub-steps' code: a lone sphere 14.4 us otherwise, 14.1)
         bool failed = hold.left > 0;
         if (__builtin_expect(failed, 0)) {
             --hold.left;
