@@ -431,9 +431,10 @@ int lbdem_dem_substeps(lbdem_dem *D, int32_t nsub, void *stream);
  * work: LBDEM_DEM_FLOW_BYTES(n) of 256-byte aligned device memory, zeroed once
  * by the caller and kept by it between calls, for one solver; D->sync must be
  * zeroed once too.  Where the form does not apply (a short periodic axis, more
- * particles than one resident wave holds, one or two sub-steps -- three of 9 to
- * 16 particles --, no workspace, LBDEM_DEM_KERNELS set in the environment) this
- * is lbdem_dem_substeps. */
+ * particles than one resident wave holds, one or two sub-steps -- only one of
+ * one or two particles or, of up to 16, with periodic images; three of 9 to 16
+ * without --, no workspace, LBDEM_DEM_KERNELS set in the environment) this is
+ * lbdem_dem_substeps. */
 #define LBDEM_DEM_FLOW_BYTES(n) (256 + 512 * (size_t)(n))
 int lbdem_dem_substeps_flow(lbdem_dem *D, int32_t nsub, void *work, void *stream);
 

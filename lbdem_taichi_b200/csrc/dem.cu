@@ -946,15 +946,19 @@ constexpr int COOP_MIN_SUBSTEPS = 3;
 // for one sub-step against 18 / 21, 29 / 48 for two against 26 / 40, 31 / 50
 // for three against 35 / 59).
 constexpr int FLOW_MIN_SUBSTEPS = 3;
-// In one block (16 particles) the two-phase form needs no grid barrier, and one
-// to three sub-steps are the shorter by it where particles touch: particles
-// apart / touching, two-phase against this form, us: one sub-step of 1, 8 and 16
-// particles 6.3 / 6.3, 6.7 / 6.9, 6.4 / 7.1 against 8.1 / 10.9, 9.7 / 20.7, 10.2
-// / 23.3; two 11.0 / 10.7, 11.4 / 11.3, 11.1 / 10.6 against 9.1 / 12.0, 10.6 /
-// 22.9, 10.7 / 25.2; three 14.4 / 15.0, 15.9 / 16.6, 16.6 / 18.0 against 9.6 /
-// 11.9, 11.0 / 24.0, 11.4 / 26.8; ten 43 / 41, 49 / 42, 48 / 55 against 15 / 18,
-// 16 / 36, 17 / 39.
-constexpr int FLOW_MIN_ONE_BLOCK_FEW = 3, FLOW_MIN_ONE_BLOCK = 4, ONE_BLOCK_FEW = 8;
+// In one block (16 particles) the two-phase form needs no grid barrier, and a few
+// sub-steps are the shorter by it where particles touch: particles apart /
+// touching, two-phase against this form, us: one sub-step of 1, 8 and 16 particles
+// 6.3 / 6.3, 6.7 / 6.9, 6.4 / 7.1 against 8.1 / 10.9, 9.7 / 20.7, 10.2 / 23.3; two
+// of 1, 2, 8 and 16 11.0 / 10.7, 10.9 / 11.6, 11.4 / 11.3, 11.1 / 10.6 against 9.1
+// / 12.0, 9.2 / 14.2, 10.6 / 22.9, 10.7 / 25.2; three of 8 and 16 15.9 / 16.6, 16.6
+// / 18.0 against 11.0 / 24.0, 11.4 / 26.8; ten 49 / 42, 48 / 55 against 16 / 36, 17
+// / 39.  With periodic images, whose cells the two-phase form looks up in every
+// sub-step: one of 16 9.5 / 11.1 against 10.4 / 23.2, two 17.0 / 20.3 against 10.2
+// / 24.7.
+static int flow_min_one_block(const lbdem_dem *D) {
+    return D->wrap_pairs || D->n <= 2 ? 2 : D->n <= 8 ? 3 : 4;
+}
 constexpr size_t FLOW_HEADER = 256;   // workspace: two failure words (by chunk parity), the epoch, the hold, then the packets
 // After a chunk that failed, this many chunks at most go to the two-phase form
 // without a search (1, 3, 7, ... while they keep failing; FlowHold): what breaks
@@ -1806,7 +1810,7 @@ int lbdem_dem_substeps_flow(lbdem_dem *D, int32_t nsub, void *work, void *stream
     int dev = 0, nb = 0, form = -1;
     cudaGetDevice(&dev);
     if (work && D->n > 0 && nsub > 0 && (!mode || strcmp(mode, "flow") == 0)) form = flow_form(D, dev, &nb);
-    const int least = nb > 1 ? FLOW_MIN_SUBSTEPS : D->n <= ONE_BLOCK_FEW ? FLOW_MIN_ONE_BLOCK_FEW : FLOW_MIN_ONE_BLOCK;
+    const int least = nb > 1 ? FLOW_MIN_SUBSTEPS : flow_min_one_block(D);
     // (the barrier's arrival counter must stay far from wrapping)
     if (form < 0 || (!mode && nsub < least) || 8ll * nsub * nb >= (1ll << 30))
         return lbdem_dem_substeps(D, nsub, stream);

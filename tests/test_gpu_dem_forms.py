@@ -40,20 +40,22 @@ def test_bed(side, images, monkeypatch):
     assert not a.flow[24:32].any()                      # no chunk failed
 
 
-@pytest.mark.parametrize("n", [1, 8, 9, 16, 17])
+@pytest.mark.parametrize("images", [False, True])
+@pytest.mark.parametrize("n", [1, 2, 3, 8, 9, 16, 17])
 @pytest.mark.parametrize("nsub", [1, 2, 3, 4])
-def test_short_calls_of_few_particles(n, nsub, monkeypatch):
+def test_short_calls_of_few_particles(n, nsub, images, monkeypatch):
     """The default form of short calls, on either side of where one block's
-    two-phase form gives way: 3 sub-steps up to 8 particles, 4 above; more than
-    one block, 3."""
+    two-phase form gives way: 2 sub-steps of one or two particles or with
+    periodic images, 3 up to 8 particles, 4 above; more than one block, 3."""
     rng = np.random.default_rng(n)
     pos = 2.0 + 1.995 * np.stack(np.meshgrid(*[np.arange(3)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
     vel = rng.normal(0, 0.01, (n, 3))
     a, b = (make_dem((0, 24, 0, 24, 0, 24), 0.02, (0, 0, -1e-3), HertzContactConfig(0.3, 0.3, 0.9, 0.9), np.ones(n),
-                     np.full(n, 8.0), pos, vel, periodic=(True, True, False), E=1e3, wall_E=1e3) for _ in range(2))
+                     np.full(n, 8.0), pos, vel, periodic=(True, True, False), E=1e3, wall_E=1e3,
+                     compat="wrapped" if images else "reference") for _ in range(2))
     for _ in range(3):
         _run(monkeypatch, None, a, nsub)
         _run(monkeypatch, "split", b, nsub)
     _same(a, b)
-    flow = nsub >= (3 if n <= 8 or n > 16 else 4)
+    flow = nsub >= (3 if n > 16 else 2 if images or n <= 2 else 3 if n <= 8 else 4)
     assert (a.flow[16:24].cpu().numpy().view(np.uint64)[0] > 0) == flow   # the one-launch form counts its chunks
